@@ -16,6 +16,8 @@
 // tree build's, so the set of leaves each prior sums over is exact.
 #include <cub/cub.cuh>
 
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "handles.h"
@@ -160,7 +162,7 @@ constexpr int PT_BLOCK = 128;
 #define TSR_CONE_S_BLOCKS 5
 #endif
 #ifndef TSR_PRIOR_BLOCKS
-#define TSR_PRIOR_BLOCKS 1
+#define TSR_PRIOR_BLOCKS 4
 #endif
 
 // ------------------------------------------- block-expansion cone traversal
@@ -177,11 +179,13 @@ constexpr int PT_BLOCK = 128;
 // its sum is non-zero (every accepted value is >= EPSILON), so they are set
 // afterwards from the sums.
 //
-// Node records: rec[i + 7] = (first child or INVALID, leaf index or
-// REC_NOLEAF, with the node's SAMPLENESS flag in bit 31).  Children blocks
-// start at 1 + 8k (root 0, then whole blocks of 8), so a block's records
-// start on a 64-byte boundary.
+// Node records: rec[i + 7] = (first child or INVALID, leaf index, with the
+// node's SAMPLENESS flag in bit 31).  Children blocks start at 1 + 8k (root 0,
+// then whole blocks of 8), so a block's records start on a 64-byte boundary.
+// An inner node's second word holds REC_INNER with two bits of what its
+// children block has: flagged leaves, flagged inner nodes.
 constexpr uint32_t REC_FLAG = 0x80000000u, REC_NOLEAF = 0x7FFFFFFFu;
+constexpr uint32_t REC_INNER = 0x7FFFFFFCu, REC_HAS_LEAVES = 1u, REC_HAS_INNER = 2u;
 constexpr uint32_t REC_OFFSET = 7;
 
 __global__ void k_pack_rec(uint32_t nn, const uint32_t *children, const uint32_t *node_to_leaf,
@@ -189,8 +193,13 @@ __global__ void k_pack_rec(uint32_t nn, const uint32_t *children, const uint32_t
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn) return;
     uint32_t c = children[i];
-    uint32_t y = (c == INVALID) ? node_to_leaf[i] : REC_NOLEAF;
-    if (states && (states[i] & FLAG_SAMPLENESS)) y |= REC_FLAG;
+    uint32_t y = (c == INVALID) ? node_to_leaf[i] : REC_INNER;
+    if (states) {
+        if (states[i] & FLAG_SAMPLENESS) y |= REC_FLAG;
+        if (c != INVALID)
+            for (uint32_t k = 0; k < 8; ++k)
+                if (states[c + k] & FLAG_SAMPLENESS) y |= children[c + k] == INVALID ? REC_HAS_LEAVES : REC_HAS_INNER;
+    }
     rec[i + REC_OFFSET] = make_uint2(c, y);
 }
 
@@ -231,15 +240,13 @@ __global__ void k_prior_needed(uint32_t nl, const uint8_t *pred, const double *e
 // same margin): DMC snaps a vertex to the end of an edge whose value is
 // within EPSILON of zero, and a negative leaf's value is -EPSILON, so that
 // side is all the mesh takes from a positive leaf's value.
-__global__ void k_certify(uint32_t n, const uint32_t *list, const double *esum, const double *ssum,
-                          const double2 *bounds, const double *cone_count, uint8_t *pred, uint8_t *need,
-                          unsigned long long *certified) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_certify(uint32_t nl, const double *esum, const double *ssum, const double2 *bounds,
+                          const double *cone_count, uint8_t *pred, uint8_t *need, unsigned long long *certified) {
+    const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     bool ok = false;
-    if (i < n) {
-        const uint32_t l = list[i];
+    if (l < nl && need[l] == NEED_CERTIFY) {
         const double e = esum[l], s = ssum[l];
-        const double2 b = bounds[i];
+        const double2 b = bounds[l];
         const double margin = 1e-9 * (s + e);
         const double at_hi = (1.0 - b.y) * s - b.y * e, at_lo = (1.0 - b.x) * s - b.x * e;
         const bool pos = at_hi > margin;
@@ -582,29 +589,13 @@ __global__ void k_repair_mark(uint32_t nl, const uint32_t *nb_off, const uint32_
     }
 }
 
-__global__ void k_flag_equal(uint32_t n, const uint8_t *v, uint8_t value, uint8_t *flag) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flag[i] = v[i] == value ? 1 : 0;
-}
-
-__global__ void k_set_needed(uint32_t n, const uint32_t *list, uint8_t *need) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) need[list[i]] = 1;
-}
-
-// Depth of every listed leaf (list == null: leaves 0 .. n-1) as a sort key.
-__global__ void k_leaf_depth_keys(uint32_t n, const uint32_t *list, const uint32_t *leaf_node, const uint8_t *depth,
-                                  uint32_t *keys, uint32_t *vals) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t l = list ? list[i] : i;
-    keys[i] = depth[leaf_node[l]];
-    vals[i] = l;
-}
-
-__global__ void k_iota(uint32_t n, uint32_t *out) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = i;
+// The marked leaves become queried ones, counted.
+__global__ void k_set_needed(uint32_t nl, const uint8_t *mark, uint8_t *need, uint32_t *count) {
+    const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool m = l < nl && mark[l];
+    if (m) need[l] = NEED_QUERY;
+    const unsigned b = __ballot_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(count, (uint32_t)__popc(b));
 }
 
 // A leaf carries a type's flag exactly when it received a kernel of that type.
@@ -656,7 +647,7 @@ constexpr int PK = 8;
 
 __global__ void k_prior_sums(uint32_t lo, uint32_t hi, uint32_t nn, const uint32_t *order,
                              const uint32_t *children, const uint32_t *node_to_leaf, const uint32_t *states,
-                             const double *elen, const double *slen, double2 *psum) {
+                             const double *elen, const double *slen, double2 *psum, int *nonfinite) {
     uint32_t i = lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= hi) return;
     uint32_t n = order[i];
@@ -666,6 +657,7 @@ __global__ void k_prior_sums(uint32_t lo, uint32_t hi, uint32_t nn, const uint32
         if (states[n] & FLAG_SAMPLENESS) {
             uint32_t l = node_to_leaf[n];
             v = make_double2(elen[l], slen[l]);
+            if (!isfinite(v.x) || !isfinite(v.y)) *nonfinite = 1;
         }
         for (int k = 0; k < PK; ++k) psum[(size_t)k * nn + n] = v;
         return;
@@ -703,221 +695,493 @@ __device__ inline bool box_inside_sphere(const D3 &mn, double sz, const D3 &c, d
     return dx * dx + dy * dy + dz * dz <= r * r * (1.0 - 1e-9);
 }
 
+// Children block b (nodes 1 + 8b .. 8 + 8b): the parent's corner on the
+// lattice of 2^24 cells along the root's edge, and the children's depth.  Any
+// corner down to depth 24 is a whole number below 2^24 there, exact in FP32.
+constexpr uint32_t LATTICE_DEPTH = 24;
+
+__global__ void k_block_corners(uint32_t nb, const uint32_t *parents, const uint8_t *depth, float4 *out) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nb) return;
+    const uint32_t first = 1 + 8 * b, d = depth[first];
+    uint32_t x = 0, y = 0, z = 0, node = parents[first];
+    for (uint32_t k = d - 1; k > 0; --k) {   // the node at depth k is child (node - 1) & 7 of its parent
+        const uint32_t c = (node - 1) & 7u;
+        if (k <= LATTICE_DEPTH) {
+            const uint32_t step = LATTICE_DEPTH - k;
+            x |= (c & 1u) << step;
+            y |= ((c >> 1) & 1u) << step;
+            z |= ((c >> 2) & 1u) << step;
+        }
+        node = parents[node];
+    }
+    out[b] = make_float4((float)x, (float)y, (float)z, __uint_as_float(d));
+}
+
+// Sort keys of the children blocks: the depth of the block's nodes.
+__global__ void k_block_depth_keys(uint32_t nb, const uint8_t *depth, uint32_t *keys, uint32_t *vals) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nb) return;
+    keys[b] = depth[1 + 8 * b];
+    vals[b] = b;
+}
+
+// Blocks of `list` that hold a leaf whose sel[leaf] == value, and how many such leaves there are.
+__global__ void k_blocks_with(uint32_t nb, const uint32_t *list, const uint2 *rec, const uint8_t *sel, uint8_t value,
+                              uint8_t *flag, uint32_t *leaves) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t count = 0;
+    if (i < nb) {
+        const uint2 *r = rec + 1 + 8 * list[i] + REC_OFFSET;
+        for (int c = 0; c < 8; ++c)
+            if (r[c].x == INVALID && sel[r[c].y & REC_NOLEAF] == value) ++count;
+        flag[i] = count ? 1 : 0;
+    }
+    for (int o = 16; o; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
+    if ((threadIdx.x & 31) == 0 && count) atomicAdd(leaves, count);
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// What the prior queries read of the tree and the field.
+struct PriorIn {
+    uint32_t nn;
+    const uint32_t *parents;
+    const D3 *nmin;             // FP64 corners, for the tests that need them
+    const uint2 *rec;
+    const float4 *blocks;
+    const double2 *psum;
+    const int *nonfinite;       // != 0: a leaf's cone length is infinite or NaN
+    double root_size, rel_radius;
+    double corner_error;        // bound of an FP64 corner's or centre's distance from its lattice point
+    bool deep;                  // deeper than the lattice: corners from nmin
+    bool whole_radius;          // eight radii are a whole number, small enough for exact FP32 squares
+};
+
+constexpr int PP_STACK = 28 * MAX_TREE_DEPTH + 32;   // a step pops four blocks and pushes at most 32
+constexpr int PP_LEAVES = 64;   // blocks whose leaves wait; worked off when fewer than 32 are free
+constexpr int PP_TIES = 64;     // leaves that touch a sphere; likewise
+constexpr int PP_WARPS = 4;
+
 // Occupancy::computePriors (Occupancy.cpp:530-568) with a
 // SphereNodeStatesChecker (SphereNodeStatesChecker.cpp:28-36).  The set of
-// summed leaves is the reference's: SAMPLENESS-flagged leaves at most three
-// levels below the query leaf whose box meets the sphere (the exact FP64
-// test); subtrees wholly inside the sphere are added from psum, whose row 0
-// of a leaf is the leaf's own (emptiness, sampleness) cone-length pair.
+// leaves a query sums is the reference's: SAMPLENESS-flagged leaves at most
+// three levels below the query leaf whose box meets the sphere; subtrees
+// wholly inside the sphere are added from psum, whose row 0 is a flagged
+// leaf's own (emptiness, sampleness) cone-length pair and zero elsewhere.
 //
-// Run by persistent threads over the traversal records of the cone passes,
-// expanding one node per step: its eight children's records come in one
-// 64-byte line and their FP64 boxes are derived from the parent's corner with
-// the tree build's own recurrence (child_coords, exact), so no node geometry
-// is loaded inside the loop.
+// One warp answers the queries of the up to eight leaves of a children block
+// together: they have one size, their centres are one leaf size apart, and
+// their radius is 25 of it, so their spheres take in nearly the same nodes.
+// Two kinds of steps take four children blocks each, one node a lane, so the
+// records, corners and cone lengths of a block arrive in whole lines:
+//  * inner nodes are decided for the eight spheres at once: inside all (a row
+//    of psum is added), outside all, or their children block is next -- its
+//    inner nodes on the stack, its leaves on a second list;
+//  * leaves are tested against each of the eight spheres.  Their centres are a
+//    2 x 2 x 2 lattice, so the squared distances are sums of two terms per
+//    axis, and every lane keeps the eight sums of the leaves it met; they are
+//    added across the warp once, at the end.
 //
-// BOUNDS (the pruned field's sign certificates): a node that straddles the
-// sphere at depth >= the query leaf's depth - coarse_up is not descended;
-// its whole subtree row is added to an undecided pair (eU, sU) instead, so
-// the query ends early with eL <= E <= eL + eU and sL <= S <= sL + sU for
-// the exact sums E, S, and writes bounds[i] = (eL / (eL + sL + sU),
-// (eL + eU) / (eL + eU + sL)) around the prior E / (E + S).
-template <bool BOUNDS>
-__global__ void __launch_bounds__(PT_BLOCK, TSR_PRIOR_BLOCKS) k_priors_x(uint32_t nl, uint32_t nn, const uint32_t *list,
-                                                      const uint32_t *leaf_node, const D3 *leaf_min,
-                                                      const uint8_t *depth, const D3 *nmin, const uint2 *rec,
-                                                      const double2 *psum, double root_size, double rel_radius,
-                                                      double *prior, unsigned long long *next_leaf,
-                                                      unsigned long long *visits, int *err, double2 *bounds,
-                                                      uint32_t coarse_up) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31;
-    uint64_t st[MAX_TREE_DEPTH];   // children block | mask << 32 | depth << 40
-    int sp = 0;
-    bool have = false, active = false, done = false;
-    uint32_t x_c0 = 0, x_d = 0;
-    D3 x_min{0.0, 0.0, 0.0};
-    uint32_t l = 0, max_depth = 0, qi = 0, stop_depth = 0;
-    D3 center{0.0, 0.0, 0.0};
-    double radius = 0.0, eL = 0.0, sL = 0.0, eU = 0.0, sU = 0.0;
-    float r2f = 0.0f;
-    unsigned long long nvis = 0;
-    auto add_row = [&](uint32_t n, uint32_t k) {
-        double2 v = psum[(size_t)k * nn + n];
-        eL += v.x;
-        sL += v.y;
+// Lengths are in eighths of the query leaf's size, in the frame of the
+// block's centre: every corner is a whole number, and the FP32 distances are
+// exact wherever they decide anything.  A distance within `tol` of the radius
+// (in practice a box that touches a sphere) is decided by the FP64 boxes, as
+// the reference does.
+//
+// Measured, all queries of the field: 493 -> 183 ms at 16M held-out samples
+// (7.6M leaves), 34 -> 14.5 ms at 4M CSG samples, 1.5 -> 0.5 ms at 4k sphere
+// samples.  A query per lane read eight records and eight psum rows of its own
+// per expansion, 128 + 256 cache lines a warp's step, and the L1 passed 0.7
+// child tests a clock and SM; here the lines are shared, a test costs 12 of a
+// lane's instructions, and what bounds it is the issue of four warps per
+// scheduler (126 registers; five warps spill and are no faster).  The eight
+// spheres test 1.6 times the boxes one does.
+//
+// BOUNDS (the pruned field's sign certificates): a node that straddles a
+// query's sphere at depth >= the query leaf's depth - coarse_up is not
+// descended; its whole subtree row is added to an undecided pair (eU, sU)
+// instead, so the query ends early with eL <= E <= eL + eU and
+// sL <= S <= sL + sU for the exact sums E, S, and writes
+// bounds[leaf] = (eL / (eL + sL + sU), (eL + eU) / (eL + eU + sL)) around the
+// prior E / (E + S).
+struct Packet {   // the block of queries a warp works on
+    float scale, cx, cy, cz;   // lattice cells -> eighths of the query leaf's size, packet frame
+    double size;
+    float ea;                  // bound of a corner's distance from its lattice point
+    uint32_t q0, max_depth;
+};
+
+struct Box {
+    float x, y, z, h;   // centre, half edge length
+    float e;            // bound of a corner's error
+};
+
+// A node's box from its block's corner and its size.
+__device__ __forceinline__ Box box_of(const PriorIn &in, const Packet &P, uint32_t node, float lx, float ly, float lz,
+                                      float sz, float bx, float by, float bz) {
+    Box b;
+    b.h = 0.5f * sz;
+    b.e = P.ea;
+    if (!in.deep) {
+        b.x = fmaf(bx, sz, lx) + b.h;
+        b.y = fmaf(by, sz, ly) + b.h;
+        b.z = fmaf(bz, sz, lz) + b.h;
+    } else {
+        const D3 m = in.nmin[node], o = in.nmin[in.parents[P.q0]];
+        const double k = 8.0 / P.size;
+        b.x = (float)(((m.x - o.x) - P.size) * k) + b.h;
+        b.y = (float)(((m.y - o.y) - P.size) * k) + b.h;
+        b.z = (float)(((m.z - o.z) - P.size) * k) + b.h;
+        b.e += 4e-7f * (fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fabsf(b.z)) + sz);
+    }
+    return b;
+}
+
+// Bound of the FP32 error of a squared distance near the radius.
+__device__ __forceinline__ float distance_error(float e, float ru) {
+    return e > 0.01f * ru ? INFINITY : 4.0f * ru * e + 4e-7f * ru * ru;
+}
+
+// Four times the squared distances of the box from the eight centres (at +-4
+// on each axis), less r4 = 4 r^2.  t + |t| = 2 max(t, 0) keeps the work on the
+// FMA pipe; the minimum would go to the ALU, which has half its rate.
+__device__ __forceinline__ void near_distances(const Box &b, float r4, float *s) {
+    auto sq = [&](float c, float less) {
+        const float t = fabsf(c) - b.h, u = t + fabsf(t);
+        return fmaf(u, u, less);
     };
+    const float X0 = sq(b.x + 4.0f, 0.0f), X1 = sq(b.x - 4.0f, 0.0f), Y0 = sq(b.y + 4.0f, -r4),
+                Y1 = sq(b.y - 4.0f, -r4), Z0 = sq(b.z + 4.0f, 0.0f), Z1 = sq(b.z - 4.0f, 0.0f);
+    const float xy[4] = {X0 + Y0, X1 + Y0, X0 + Y1, X1 + Y1};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] = xy[q & 3] + ((q & 4) ? Z1 : Z0);
+}
+
+// The same of the box's far corner.
+__device__ __forceinline__ void far_distances(const Box &b, float r4, float *s) {
+    auto sq = [&](float c, float less) {
+        const float t = 2.0f * (fabsf(c) + b.h);
+        return fmaf(t, t, less);
+    };
+    const float X0 = sq(b.x + 4.0f, 0.0f), X1 = sq(b.x - 4.0f, 0.0f), Y0 = sq(b.y + 4.0f, -r4),
+                Y1 = sq(b.y - 4.0f, -r4), Z0 = sq(b.z + 4.0f, 0.0f), Z1 = sq(b.z - 4.0f, 0.0f);
+    const float xy[4] = {X0 + Y0, X1 + Y0, X0 + Y1, X1 + Y1};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q] = xy[q & 3] + ((q & 4) ? Z1 : Z0);
+}
+
+// e += v.x / 128, s += v.y / 128 where d < 0, without a predicate: a predicated
+// FP64 addition becomes four selects on the half-rate ALU before it (58 of a
+// step's 137 instructions).  sat(-d BIG) is 1.0f or 0.0f, and the bits of
+// 1.0f over a zero word are the double 2^-7: an exact product and one rounding.
+// The values must be finite.
+__device__ __forceinline__ void add_where_negative(float d, const double2 &v, double &e, double &s) {
+    const double w = __hiloint2double(__float_as_int(__saturatef(d * -1e30f)), 0);
+    e = fma(v.x, w, e);
+    s = fma(v.y, w, s);
+}
+constexpr double PP_UNIT = 128.0;
+
+// The reference's decision of query q of the packet about a node whose FP32
+// distance leaves it open: its box and every box above it meet the sphere (1),
+// and the box is inside (2).  A box that touches the sphere can pass while the
+// box around it, whose far corner is rounded differently, does not; so the
+// boxes above are tested too, up to the first that clearly meets.
+__device__ __noinline__ int exact_place(const PriorIn *in_p, const Packet *P, uint32_t q, uint32_t node) {
+    const PriorIn &in = *in_p;
+    const float ru = 8.0f * (float)in.rel_radius;
+    const D3 qm = in.nmin[P->q0 + q];
+    const double hs = dmul(0.5, P->size), radius = dmul(P->size, in.rel_radius);
+    const D3 c{dadd(qm.x, hs), dadd(qm.y, hs), dadd(qm.z, hs)};
+    uint32_t n = node;
+    bool inside = false;
     while (true) {
-        if (!have && sp > 0) {
-            uint64_t e = st[sp - 1];
-            uint32_t m = (uint32_t)(e >> 32) & 0xFFu;
-            uint32_t node = (uint32_t)e + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1;
-            if (m) st[sp - 1] = (e & ~(0xFFull << 32)) | ((uint64_t)m << 32); else --sp;
-            x_c0 = __ldg(&rec[node + REC_OFFSET]).x;
-            x_min = nmin[node];   // the build's own FP64 corner of that node
-            x_d = (uint32_t)(e >> 40) + 1;
-            have = true;
+        const float4 B = n ? in.blocks[(n - 1) >> 3] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t d = n ? __float_as_uint(B.w) : 0;
+        const D3 mn = in.nmin[n];
+        const double sz = ldexp(in.root_size, -(int)d);
+        if (!sphere_meets_box(mn, D3{dadd(mn.x, sz), dadd(mn.y, sz), dadd(mn.z, sz)}, c, radius)) return 0;
+        if (n == node) inside = box_inside_sphere(mn, sz, c, radius);
+        if (d == 0) break;
+        n = in.parents[n];
+        if (in.deep) continue;
+        // the parent's box: corner B, twice the edge length
+        const float h = __uint_as_float((127u + P->max_depth - d) << 23);
+        const float x = fabsf(fmaf(B.x, P->scale, P->cx) + h + ((q & 1u) ? -4.0f : 4.0f)) - h;
+        const float y = fabsf(fmaf(B.y, P->scale, P->cy) + h + ((q & 2u) ? -4.0f : 4.0f)) - h;
+        const float z = fabsf(fmaf(B.z, P->scale, P->cz) + h + ((q & 4u) ? -4.0f : 4.0f)) - h;
+        const float X = fmaxf(x, 0.0f), Y = fmaxf(y, 0.0f), Z = fmaxf(z, 0.0f);
+        if (X * X + Y * Y + Z * Z - ru * ru < -distance_error(P->ea, ru)) break;
+    }
+    return inside ? 2 : 1;
+}
+
+struct PriorWarp {
+    Packet packet;
+    float4 leaf_box[PP_LEAVES];     // a waiting block's corner (packet frame) and its nodes' size
+    uint32_t leaf_block[PP_LEAVES];
+    uint32_t tie_node[PP_TIES];     // a leaf, and the queries whose sphere it touches
+    uint8_t tie_mask[PP_TIES];
+    uint32_t stack[PP_STACK];
+};
+
+template <bool BOUNDS>
+__global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
+    k_priors(uint32_t nblocks, const uint32_t *list, const __grid_constant__ PriorIn in, const uint8_t *sel,
+             uint8_t value, double *prior, double2 *bounds, uint32_t coarse_up, unsigned long long *next_block,
+             unsigned long long *visits, int *err) {
+    const unsigned FULL = 0xffffffffu;
+    __shared__ PriorWarp shared[PP_WARPS];
+    PriorWarp &w = shared[threadIdx.x >> 5];
+    const Packet &P = w.packet;
+    const unsigned lane = threadIdx.x & 31, below = (1u << lane) - 1u, ci = lane & 7u;
+    const int quarter = (int)(lane >> 3);
+    const float bx = (float)(ci & 1u), by = (float)((ci >> 1) & 1u), bz = (float)(ci >> 2);
+    const float ru = 8.0f * (float)in.rel_radius, r2 = ru * ru, r4 = 4.0f * r2;
+    const bool finite = *in.nonfinite == 0;
+    unsigned long long nvis = 0;
+    while (true) {
+        unsigned long long bi = 0;
+        if (lane == 0) bi = atomicAdd(next_block, 1ull);
+        bi = __shfl_sync(FULL, bi, 0);
+        if (bi >= nblocks) break;
+        const uint32_t qb = list[bi];
+        const uint2 qrec = __ldg(&in.rec[1 + 8 * qb + ci + REC_OFFSET]);
+        const uint32_t qleaf = qrec.y & REC_NOLEAF;
+        const bool wanted = qrec.x == INVALID && (!sel || sel[qleaf] == value);
+        const unsigned mask = __ballot_sync(FULL, wanted) & 0xFFu;
+        if (!mask) continue;
+        const float4 Q = __ldg(&in.blocks[qb]);
+        const uint32_t pd = __float_as_uint(Q.w);
+        const uint2 root = __ldg(&in.rec[REC_OFFSET]);
+        int sp = 0, waiting = 0, ties = 0;
+        if (lane == 0) {
+            Packet k;
+            k.q0 = 1 + 8 * qb;
+            k.max_depth = pd + MAX_DEPTH_DIFFERENCE;
+            k.size = ldexp(in.root_size, -(int)pd);
+            k.scale = ldexpf(1.0f, (int)k.max_depth - (int)LATTICE_DEPTH);
+            const float half = ldexpf(1.0f, (int)LATTICE_DEPTH - (int)pd);
+            k.cx = -(Q.x + half) * k.scale;
+            k.cy = -(Q.y + half) * k.scale;
+            k.cz = -(Q.z + half) * k.scale;
+            k.ea = (float)(in.corner_error / k.size) * 8.0f;
+            w.packet = k;
+            w.stack[0] = w.leaf_block[0] = 0;
+            w.leaf_box[0] = make_float4(k.cx, k.cy, k.cz, __uint_as_float((126u + k.max_depth) << 23));
         }
-        if (!have && active) {   // query finished
-            if (BOUNDS)
-                bounds[qi] = make_double2(eL / (eL + sL + sU), (eL + eU) / (eL + eU + sL));
-            else
-                prior[l] = eL / (eL + sL);
-            active = false;
+        if (root.y & REC_FLAG) {   // the root's children (the root itself holds every centre)
+            if (root.y & REC_HAS_INNER) sp = 1;
+            if (root.y & REC_HAS_LEAVES) waiting = 1;
         }
-        bool need = !have && !done;
-        unsigned nm = __ballot_sync(FULL, need);
-        if (nm) {
-            int leader = __ffs(nm) - 1;
-            unsigned long long b = 0;
-            if ((int)lane == leader) b = atomicAdd(next_leaf, (unsigned long long)__popc(nm));
-            b = __shfl_sync(FULL, b, leader);
-            if (need) {
-                uint64_t i = b + __popc(nm & ((1u << lane) - 1u));
-                if (i >= nl) {
-                    done = true;
-                } else {
-                    qi = (uint32_t)i;
-                    l = list ? list[i] : (uint32_t)i;
-                    uint32_t node = leaf_node[l];
-                    uint32_t ld = depth[node];
-                    stop_depth = ld > coarse_up + 1 ? ld - coarse_up : 1;
-                    double size = size_at(root_size, ld);
-                    D3 mn = leaf_min[l];
-                    double half = dmul(0.5, size);
-                    center = D3{dadd(mn.x, half), dadd(mn.y, half), dadd(mn.z, half)};
-                    radius = dmul(size, rel_radius);
-                    r2f = (float)dmul(radius, radius);
-                    max_depth = ld + MAX_DEPTH_DIFFERENCE;
-                    eL = sL = eU = sU = 0.0;
-                    active = true;
-                    // the root (SphereNodeStatesChecker on node 0)
-                    uint2 r0 = __ldg(&rec[REC_OFFSET]);
-                    D3 bmn = nmin[0];
-                    D3 bmx{dadd(bmn.x, root_size), dadd(bmn.y, root_size), dadd(bmn.z, root_size)};
-                    if ((r0.y & REC_FLAG) && aabb_sphere(bmn, bmx, center, radius)) {
-                        if (max_depth < (uint32_t)PK && box_inside_sphere(bmn, root_size, center, radius)) {
-                            add_row(0, max_depth);
-                        } else if (r0.x == INVALID) {
-                            add_row(0, 0);
-                        } else if (1 <= max_depth) {
-                            x_c0 = r0.x;
-                            x_min = bmn;
-                            x_d = 1;
-                            have = true;
+        double aE[8], aS[8], uE[BOUNDS ? 8 : 1], uS[BOUNDS ? 8 : 1], allE = 0.0, allS = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) aE[q] = aS[q] = 0.0;
+        if (BOUNDS) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) uE[q] = uS[q] = 0.0;
+        }
+        uint32_t tested = 0;
+        __syncwarp();
+        // whole-numbered distances: undecided only when zero
+        const bool whole = in.whole_radius && !in.deep && 4.0f * ru * P.ea < 0.125f;
+        while (sp > 0 || waiting > 0 || ties > 0) {
+            if (ties > PP_TIES - 32 || (sp == 0 && waiting == 0)) {
+                // ---- leaves that touch a sphere: a lane each
+                for (int j = lane; j < ties; j += 32) {
+                    const uint32_t node = w.tie_node[j];
+                    unsigned met = 0;
+                    for (unsigned rest = w.tie_mask[j]; rest; rest &= rest - 1) {
+                        const uint32_t q = __ffs(rest) - 1;
+                        if (exact_place(&in, &P, q, node)) met |= 1u << q;
+                    }
+                    const double2 v = __ldg(&in.psum[node]);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if ((met >> q) & 1u) {
+                            aE[q] += v.x / PP_UNIT;
+                            aS[q] += v.y / PP_UNIT;
                         }
+                }
+                ties = 0;
+                __syncwarp();
+                continue;
+            }
+            if (waiting > PP_LEAVES - 32 || sp == 0) {
+                // ---- the leaves of the waiting blocks
+                do {
+                    const bool valid = quarter < waiting;
+                    const int at = valid ? waiting - 1 - quarter : 0;
+                    const uint32_t node = 1 + 8 * w.leaf_block[at] + ci;
+                    const float4 B = w.leaf_box[at];
+                    double2 v = make_double2(0.0, 0.0);
+                    if (valid) v = __ldg(&in.psum[node]);
+                    const Box box = box_of(in, P, node, B.x, B.y, B.z, B.w, bx, by, bz);
+                    float s[8];
+                    near_distances(box, r4, s);
+                    bool unsure;
+                    if (whole) {
+                        float product = s[0];
+#pragma unroll
+                        for (int q = 1; q < 8; ++q) product *= s[q];
+                        unsure = !(fabsf(product) > 0.0f);
+                    } else {
+                        float least = fabsf(s[0]);
+#pragma unroll
+                        for (int q = 1; q < 8; ++q) least = fminf(least, fabsf(s[q]));
+                        unsure = !(least > 4.0f * distance_error(box.e, ru));
+                    }
+                    unsure = unsure && (v.x != 0.0 || v.y != 0.0);
+                    const unsigned um = __ballot_sync(FULL, unsure);
+                    if (unsure) {   // decided later, not met here
+                        const float tol = 4.0f * distance_error(box.e, ru);
+                        unsigned ask = 0;
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (!(fabsf(s[q]) > tol)) {
+                                ask |= 1u << q;
+                                s[q] = 1.0f;
+                            }
+                        const int j = ties + __popc(um & below);
+                        w.tie_node[j] = node;
+                        w.tie_mask[j] = (uint8_t)(ask & mask);
+                    }
+                    ties += __popc(um);
+                    if (finite) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) add_where_negative(s[q], v, aE[q], aS[q]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (s[q] < 0.0f) {
+                                aE[q] += v.x / PP_UNIT;
+                                aS[q] += v.y / PP_UNIT;
+                            }
+                    }
+                    tested += 32;
+                    waiting -= 4;
+                } while ((waiting >= 4 || (waiting > 0 && sp == 0)) && ties <= PP_TIES - 32);
+                if (waiting < 0) waiting = 0;
+                __syncwarp();
+                continue;
+            }
+            // ---- the inner nodes of the blocks on top of the stack
+            const int take = sp < 4 ? sp : 4;
+            const bool valid = quarter < take;
+            const uint32_t b = w.stack[sp - 1 - (valid ? quarter : 0)], node = 1 + 8 * b + ci;
+            sp -= take;
+            tested += 8 * take;
+            const uint2 r = __ldg(&in.rec[node + REC_OFFSET]);
+            const float4 B = __ldg(&in.blocks[b]);
+            bool next = false;
+            float4 corner = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (valid && r.x != INVALID && (r.y & REC_FLAG)) {
+                const uint32_t d = __float_as_uint(B.w), k = P.max_depth - d;
+                const Box box = box_of(in, P, node, fmaf(B.x, P.scale, P.cx), fmaf(B.y, P.scale, P.cy),
+                                       fmaf(B.z, P.scale, P.cz), __uint_as_float((127u + k) << 23), bx, by, bz);
+                const float m = 4.0f + box.h + box.e;
+                const float fx = fabsf(box.x) + m, fy = fabsf(box.y) + m, fz = fabsf(box.z) + m;
+                const float nx = fmaxf(fabsf(box.x) - m, 0.0f), ny = fmaxf(fabsf(box.y) - m, 0.0f),
+                            nz = fmaxf(fabsf(box.z) - m, 0.0f);
+                const bool apart = nx * nx + ny * ny + nz * nz > r2 * (1.0f + 1e-6f);
+                const bool inside = fx * fx + fy * fy + fz * fz < r2 * (1.0f - 2e-6f);
+                if (inside && k < (uint32_t)PK) {
+                    const double2 row = in.psum[(size_t)k * in.nn + node];
+                    allE += row.x;
+                    allS += row.y;
+                } else if (!apart) {
+                    if (BOUNDS && d >= (pd > coarse_up + 1 ? pd - coarse_up : 1)) {   // k <= 3 + coarse_up < PK there
+                        const double2 row = in.psum[(size_t)k * in.nn + node];
+                        const float tol = 4.0f * distance_error(box.e, ru);
+                        float s[8], f[8];
+                        near_distances(box, r4, s);
+                        far_distances(box, r4, f);
+                        unsigned ask = 0, met = 0, in_it = 0;
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            if (!(fabsf(s[q]) > tol) || !(fabsf(f[q]) > tol)) ask |= 1u << q;
+                            if (s[q] < 0.0f) met |= 1u << q;
+                            if (f[q] < 0.0f) in_it |= 1u << q;
+                        }
+                        for (unsigned rest = ask & mask; rest; rest &= rest - 1) {
+                            const uint32_t q = __ffs(rest) - 1;
+                            const int place = exact_place(&in, &P, q, node);
+                            met = (met & ~(1u << q)) | (place > 0 ? 1u << q : 0u);
+                            in_it = (in_it & ~(1u << q)) | (place > 1 ? 1u << q : 0u);
+                        }
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            if (!((met >> q) & 1u)) continue;
+                            if ((in_it >> q) & 1u) {
+                                aE[q] += row.x / PP_UNIT;
+                                aS[q] += row.y / PP_UNIT;
+                            } else {
+                                uE[q] += row.x;
+                                uS[q] += row.y;
+                            }
+                        }
+                    } else {
+                        next = d < P.max_depth;
+                        corner = make_float4(box.x - box.h, box.y - box.h, box.z - box.h, box.h);
                     }
                 }
             }
-        }
-        if (__all_sync(FULL, done && !have && sp == 0 && !active)) break;
-        if (!have) continue;
-        have = false;
-        if ((x_c0 & 7u) != 1u || x_c0 > 0xFFFFFFF0u) {
-            atomicExch(err, 3);
-            continue;
-        }
-        const uint4 *line = reinterpret_cast<const uint4 *>(rec + x_c0 + REC_OFFSET);
-        uint4 q0 = __ldg(line), q1 = __ldg(line + 1), q2 = __ldg(line + 2), q3 = __ldg(line + 3);
-        const uint32_t rx[8] = {q0.x, q0.z, q1.x, q1.z, q2.x, q2.z, q3.x, q3.z};
-        const uint32_t ry[8] = {q0.y, q0.w, q1.y, q1.w, q2.y, q2.w, q3.y, q3.w};
-        const double cs = ldexp(root_size, -(int)x_d);
-        const uint32_t d = x_d;
-        const bool can_descend = d + 1 <= max_depth;
-        const bool can_add = d <= max_depth && max_depth - d < (uint32_t)PK;
-        uint32_t mask = 0;
-        nvis += 8;
-        if (d <= max_depth) {
-            // Every test for every child without branches; only the outcome
-            // (a row to add, or a child to descend into) is conditional.  The
-            // exact FP64 tests run only where an FP32 estimate in the query
-            // centre's frame cannot decide: its error is bounded by e_a per
-            // axis (rounding of the frame offset and of two FP32 adds) plus
-            // 4e-7 of the squared distances, and a decision needs a margin
-            // of 1e-6 r^2 beyond that.  The rows of all eight children are
-            // loaded before any is added, so their L2 latencies overlap
-            // (adding 0 for the others is exact).
-            const float csf = (float)cs;
-            const float rx0 = (float)dsub(x_min.x, center.x), ry0 = (float)dsub(x_min.y, center.y),
-                        rz0 = (float)dsub(x_min.z, center.z);
-            const float ex = 4e-7f * (fabsf(rx0) + 2.0f * csf), ey = 4e-7f * (fabsf(ry0) + 2.0f * csf),
-                        ez = 4e-7f * (fabsf(rz0) + 2.0f * csf);
-            // Every child reads row krow: an added subtree needs row
-            // max_depth - d (< PK wherever one is added), and a leaf's rows
-            // are all equal, so the eight children's pairs come from one
-            // 128-byte line.
-            const uint32_t krow = max_depth - d < (uint32_t)PK ? max_depth - d : (uint32_t)PK - 1u;
-            double2 v[8];
-            uint32_t umask = 0;
-#pragma unroll
-            for (int ci = 0; ci < 8; ++ci) {
-                const bool flagged = (ry[ci] & REC_FLAG) != 0;
-                const bool leaf = rx[ci] == INVALID;
-                const float lx = (ci & 1) ? rx0 + csf : rx0, ly = (ci & 2) ? ry0 + csf : ry0,
-                            lz = (ci & 4) ? rz0 + csf : rz0;
-                const float hx = lx + csf, hy = ly + csf, hz = lz + csf;
-                const float tx = lx > 0.0f ? lx : (hx < 0.0f ? -hx : 0.0f);
-                const float ty = ly > 0.0f ? ly : (hy < 0.0f ? -hy : 0.0f);
-                const float tz = lz > 0.0f ? lz : (hz < 0.0f ? -hz : 0.0f);
-                const float d2 = tx * tx + ty * ty + tz * tz;
-                const float b1 = 2.0f * ((tx + ex) * ex + (ty + ey) * ey + (tz + ez) * ez) + 4e-7f * d2;
-                const float fx = fmaxf(fabsf(lx), fabsf(hx)), fy = fmaxf(fabsf(ly), fabsf(hy)),
-                            fz = fmaxf(fabsf(lz), fabsf(hz));
-                const float D2 = fx * fx + fy * fy + fz * fz;
-                const float b2 = 2.0f * ((fx + ex) * ex + (fy + ey) * ey + (fz + ez) * ez) + 4e-7f * D2;
-                bool meets = d2 + b1 < r2f * (1.0f - 1e-6f);
-                bool inside = can_add && (D2 + b2 < r2f * (1.0f - 2e-6f));
-                const bool meets_unsure = !meets && !(d2 - b1 > r2f * (1.0f + 1e-6f));
-                const bool inside_unsure = can_add && !inside && !(D2 - b2 > r2f * (1.0f + 1e-6f));
-                if (flagged && (meets_unsure || ((meets || meets_unsure) && inside_unsure))) {
-                    const D3 bmn = child_coords(x_min, cs, (uint32_t)ci);
-                    const D3 bmx{dadd(bmn.x, cs), dadd(bmn.y, cs), dadd(bmn.z, cs)};
-                    meets = sphere_meets_box(bmn, bmx, center, radius);
-                    inside = can_add && box_inside_sphere(bmn, cs, center, radius);
-                }
-                meets = meets && flagged;
-                // BOUNDS: a straddling node at or below the stop depth is undecided
-                // (max_depth - d <= 3 + coarse_up < PK there)
-                const bool unc = BOUNDS && meets && !inside && !leaf && d >= stop_depth;
-                const size_t row = (size_t)krow * nn + x_c0 + ci;
-                v[ci] = (meets && (inside || leaf || unc)) ? __ldg(&psum[row]) : make_double2(0.0, 0.0);
-                if (unc) umask |= 1u << ci;
-                if (meets && !inside && !leaf && can_descend && !unc) mask |= 1u << ci;
+            const uint32_t block = (r.x - 1) >> 3;
+            const bool push = next && (r.y & REC_HAS_INNER), wait = next && (r.y & REC_HAS_LEAVES);
+            const unsigned pm = __ballot_sync(FULL, push), wm = __ballot_sync(FULL, wait);
+            if (sp + __popc(pm) > PP_STACK) {
+                if (lane == 0) atomicExch(err, 2);   // deeper than any tree
+            } else {
+                if (push) w.stack[sp + __popc(pm & below)] = block;
+                sp += __popc(pm);
             }
+            if (wait) {
+                const int j = waiting + __popc(wm & below);
+                w.leaf_block[j] = block;
+                w.leaf_box[j] = corner;
+            }
+            waiting += __popc(wm);
+            __syncwarp();
+        }
+        nvis += (unsigned long long)tested * __popc(mask);
+        allE = warp_sum(allE);
+        allS = warp_sum(allS);
+        double E = 0.0, S = 0.0, UE = 0.0, US = 0.0;
 #pragma unroll
-            for (int ci = 0; ci < 8; ++ci) {
-                if (BOUNDS && ((umask >> ci) & 1u)) {
-                    eU += v[ci].x;
-                    sU += v[ci].y;
-                } else {
-                    eL += v[ci].x;
-                    sL += v[ci].y;
-                }
+        for (int q = 0; q < 8; ++q) {
+            const double te = warp_sum(aE[q]), ts = warp_sum(aS[q]);
+            double ue = 0.0, us = 0.0;
+            if (BOUNDS) {
+                ue = warp_sum(uE[q]);
+                us = warp_sum(uS[q]);
+            }
+            if ((int)lane == q) {
+                E = PP_UNIT * te + allE;
+                S = PP_UNIT * ts + allS;
+                UE = ue;
+                US = us;
             }
         }
-        if (mask) {
-            uint32_t ci = __ffs(mask) - 1;
-            uint32_t rest = mask & (mask - 1);
-            if (rest) {
-                if (sp >= MAX_TREE_DEPTH) {
-                    atomicExch(err, 2);
-                    continue;
-                }
-                st[sp++] = (uint64_t)x_c0 | ((uint64_t)rest << 32) | ((uint64_t)d << 40);
-            }
-            uint32_t nc = rx[0];
-#pragma unroll
-            for (int k = 1; k < 8; ++k)
-                if (ci == (uint32_t)k) nc = rx[k];
-            x_min = child_coords(x_min, cs, ci);
-            x_c0 = nc;
-            x_d = d + 1;
-            have = true;
+        if (lane < 8 && wanted) {
+            if (BOUNDS)
+                bounds[qleaf] = make_double2(E / (E + S + US), (E + UE) / (E + UE + S));
+            else
+                prior[qleaf] = E / (E + S);
         }
+        __syncwarp();   // the packet is done with
     }
-    for (int o = 16; o; o >>= 1) nvis += __shfl_xor_sync(FULL, nvis, o);
     if (lane == 0 && nvis) atomicAdd(visits, nvis);
+}
+
+// A tree that is one leaf, the root: its own lengths decide.
+__global__ void k_prior_root(const double2 *psum, double *prior, double2 *bounds) {
+    const double p = psum->x / (psum->x + psum->y);
+    if (bounds) bounds[0] = make_double2(p, p);
+    else prior[0] = p;
 }
 
 // Occupancy::getOccupancy (Occupancy.cpp:570-587), FP64.
@@ -977,22 +1241,20 @@ struct Timer {
     ~Timer() { cudaEventDestroy(a); cudaEventDestroy(b); }
 };
 
-// Prior queries in order of leaf depth, coarsest first, tree order within a
+// The children blocks in order of depth, coarsest first, tree order within a
 // depth (a stable radix sort of 6-bit keys).  A coarse leaf's sphere is wide
-// and its query long; taking those first keeps the persistent lanes from
-// ending on a tail of long queries, and a warp's lanes share one radius.
-static_assert(MAX_TREE_DEPTH <= 64, "depth keys are 6 bits");
-DBuf<uint32_t> depth_ordered(uint32_t n, const uint32_t *list, const uint32_t *leaf_node, const uint8_t *depth,
-                             cudaStream_t st) {
-    DBuf<uint32_t> out(n, st);
-    if (n == 0) return out;
-    DBuf<uint32_t> k1(n, st), k2(n, st), v1(n, st);
-    k_leaf_depth_keys<<<grid_for(n, BLK), BLK, 0, st>>>(n, list, leaf_node, depth, k1.p, v1.p);
-    ::tsr::note_launch();
+// and its query long; taking those first keeps the warps from ending on a
+// tail of long queries.
+static_assert(MAX_TREE_DEPTH < 64, "depth keys are 6 bits");
+DBuf<uint32_t> depth_ordered_blocks(uint32_t nb, const uint8_t *depth, cudaStream_t st) {
+    DBuf<uint32_t> out(nb, st);
+    if (nb == 0) return out;
+    DBuf<uint32_t> k1(nb, st), k2(nb, st), v1(nb, st);
+    k_block_depth_keys<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, depth, k1.p, v1.p); ::tsr::note_launch();
     size_t tmp = 0;
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k1.p, k2.p, v1.p, out.p, (int)n, 0, 6, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k1.p, k2.p, v1.p, out.p, (int)nb, 0, 6, st));
     DBuf<uint8_t> tb(tmp, st);
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(tb.p, tmp, k1.p, k2.p, v1.p, out.p, (int)n, 0, 6, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(tb.p, tmp, k1.p, k2.p, v1.p, out.p, (int)nb, 0, 6, st));
     return out;
 }
 
@@ -1038,7 +1300,7 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
     cone_count.zero();
     DBuf<unsigned long long> accepted(5, st);   // accepted E, S; visits E, S; prior visits
     accepted.zero();
-    DBuf<int> err(1, st);
+    DBuf<int> err(2, st);   // error code, non-finite cone lengths
     err.zero();
 
     LinkIn in{t.pos.p, t.nrm.p, t.scale.p, t.conf.p, t.links.p, cams.p, t.k, cv.count,
@@ -1046,15 +1308,17 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
     TreeIn tr{t.nmin.p};
     if (!update) o.links = nlinks;
     DBuf<unsigned long long> next_link(1, st);
-    unsigned x_grid = 0, prior_grid = 0;
+    unsigned x_grid = 0, prior_grid = 0, bounds_grid = 0;
     {
         int dev = 0, sms = 0, per_sm = 0;
         TSR_CUDA(cudaGetDevice(&dev));
         TSR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cone_x<EMPTINESS>, PT_BLOCK, 0));
         x_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
-        TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_priors_x<false>, PT_BLOCK, 0));
+        TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_priors<false>, 32 * PP_WARPS, 0));
         prior_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
+        TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_priors<true>, 32 * PP_WARPS, 0));
+        bounds_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
     }
     if (nl > REC_NOLEAF) fail(TSR_ERR_OVERFLOW_U32, "leaf count must stay below 2^31 - 1 for the traversal records");
     DBuf<uint2> recs((size_t)nn + 8, st);
@@ -1131,57 +1395,82 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
         k_prior_needed<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, pred, esum, ssum, p.confidence_threshold, need.p);
         ::tsr::note_launch();
     }
-    DBuf<double2> psum;   // cumulative prior sums (kept for the pruned field's repairs)
+    DBuf<double2> psum((size_t)nn * PK, st);   // cumulative prior sums
+    for (int d = (int)t.level_start.size() - 2; d >= 0; --d) {
+        uint32_t lo = t.level_start[d], hi = t.level_start[d + 1];
+        k_prior_sums<<<grid_for(hi - lo, BLK), BLK, 0, st>>>(lo, hi, nn, t.level_order.p, t.children.p,
+                                                            t.node_to_leaf.p, o.states.p, elen, slen, psum.p, err.p + 1); ::tsr::note_launch();
+    }
+    const uint32_t nb = (nn - 1) / 8;
+    DBuf<float4> block_corners(nb, st);
+    DBuf<uint32_t> block_order = depth_ordered_blocks(nb, t.depth.p, st);
+    if (nb) {
+        k_block_corners<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, t.parents.p, t.depth.p, block_corners.p); ::tsr::note_launch();
+    }
+    PriorIn pin{nn, t.parents.p, t.nmin.p, recs.p, block_corners.p, psum.p, err.p + 1, t.root_size, p.relative_radius_for_priors,
+                0.0, t.max_depth >= LATTICE_DEPTH, false};
     {
-        // the queried leaves: all of them, or the selected ones of a pruned field
-        DBuf<uint32_t> list;
-        uint32_t nq = nl;
-        psum.alloc((size_t)nn * PK, st);
-        for (int d = (int)t.level_start.size() - 2; d >= 0; --d) {
-            uint32_t lo = t.level_start[d], hi = t.level_start[d + 1];
-            k_prior_sums<<<grid_for(hi - lo, BLK), BLK, 0, st>>>(lo, hi, nn, t.level_order.p, t.children.p,
-                                                                t.node_to_leaf.p, o.states.p, elen, slen, psum.p); ::tsr::note_launch();
+        // a corner is a sum of at most MAX_TREE_DEPTH steps, a centre one more, each rounded to half an ulp
+        double m = 0.0;
+        for (int j = 0; j < 3; ++j) m = std::max(m, std::fabs(t.root_min[j]));
+        pin.corner_error = 64.0 * 1.1102230246251565e-16 * (m + t.root_size);
+        const double r = 8.0 * p.relative_radius_for_priors;
+        pin.whole_radius = r == std::floor(r) && r <= 1024.0;
+    }
+    // the priors of all leaves (sel == null), or of those with sel[leaf] == value; returns their number
+    auto query = [&](const uint8_t *sel, uint8_t value, double2 *bounds) -> uint32_t {
+        DBuf<uint32_t> chosen;
+        const uint32_t *list = block_order.p;
+        uint32_t n = nb, leaves = nl;
+        if (nb == 0) {   // the root is the only leaf
+            if (sel && read_scalar(sel, st) != value) return 0;
+            k_prior_root<<<1, 1, 0, st>>>(psum.p, o.prior.p, bounds); ::tsr::note_launch();
+            return 1;
         }
-        if (pred) {
-            DBuf<uint32_t> ids(nl, st), nsel(1, st), clist(nl, st);
-            DBuf<uint8_t> cflag(nl, st);
-            DBuf<unsigned long long> ncert(1, st);
-            ncert.zero();
-            list.alloc(nl, st);
-            k_iota<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, ids.p); ::tsr::note_launch();
+        if (sel) {
+            DBuf<uint8_t> flag(nb, st);
+            DBuf<uint32_t> counts(2, st);   // blocks, leaves
+            counts.zero();
+            chosen.alloc(nb, st);
+            k_blocks_with<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, list, recs.p, sel, value, flag.p, counts.p + 1);
+            ::tsr::note_launch();
             size_t tmp = 0;
-            TSR_CUDA(cub::DeviceSelect::Flagged(nullptr, tmp, ids.p, need.p, list.p, nsel.p, (int)nl, st));
+            TSR_CUDA(cub::DeviceSelect::Flagged(nullptr, tmp, list, flag.p, chosen.p, counts.p, (int)nb, st));
             DBuf<uint8_t> tb(tmp, st);
-            // skip candidates: certify their signs from bounds of their priors
-            k_flag_equal<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, need.p, NEED_CERTIFY, cflag.p); ::tsr::note_launch();
-            TSR_CUDA(cub::DeviceSelect::Flagged(tb.p, tmp, ids.p, cflag.p, clist.p, nsel.p, (int)nl, st));
-            const uint32_t nc = read_scalar(nsel.p, st);
-            if (nc) {
-                clist = depth_ordered(nc, clist.p, t.leaf_node.p, t.depth.p, st);
-                DBuf<double2> bnd(nc, st);
-                next_link.zero();
-                k_priors_x<true><<<prior_grid, PT_BLOCK, 0, st>>>(nc, nn, clist.p, t.leaf_node.p, t.leaf_min.p,
-                                                                  t.depth.p, t.nmin.p, recs.p, psum.p, t.root_size,
-                                                                  p.relative_radius_for_priors, nullptr, next_link.p,
-                                                                  accepted.p + 4, err.p, bnd.p, pruner->bound_levels);
-                ::tsr::note_launch();
-                k_certify<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, clist.p, esum, ssum, bnd.p, cone_count.p,
-                                                            pred_buf.p, need.p,
-                                                            ncert.p); ::tsr::note_launch();
-                o.certified = read_scalar(ncert.p, st);
-            }
-            // every leaf still needing its prior (need 1) is queried
-            TSR_CUDA(cub::DeviceSelect::Flagged(tb.p, tmp, ids.p, need.p, list.p, nsel.p, (int)nl, st));
-            nq = read_scalar(nsel.p, st);
-            o.pruned = nl - nq;
+            TSR_CUDA(cub::DeviceSelect::Flagged(tb.p, tmp, list, flag.p, chosen.p, counts.p, (int)nb, st));
+            uint32_t h[2];
+            TSR_CUDA(cudaMemcpyAsync(h, counts.p, 8, cudaMemcpyDeviceToHost, st));
+            TSR_CUDA(cudaStreamSynchronize(st));
+            n = h[0];
+            leaves = h[1];
+            list = chosen.p;
         }
-        list = depth_ordered(nq, list.p, t.leaf_node.p, t.depth.p, st);
+        if (n == 0) return leaves;
         next_link.zero();
-        k_priors_x<false><<<prior_grid, PT_BLOCK, 0, st>>>(nq, nn, list.p, t.leaf_node.p, t.leaf_min.p, t.depth.p,
-                                                          t.nmin.p, recs.p, psum.p, t.root_size,
-                                                          p.relative_radius_for_priors, o.prior.p, next_link.p,
-                                                          accepted.p + 4, err.p, nullptr, 0);
+        if (bounds)
+            k_priors<true><<<bounds_grid, 32 * PP_WARPS, 0, st>>>(n, list, pin, sel, value, nullptr, bounds,
+                                                                  pruner->bound_levels, next_link.p, accepted.p + 4,
+                                                                  err.p);
+        else
+            k_priors<false><<<prior_grid, 32 * PP_WARPS, 0, st>>>(n, list, pin, sel, value, o.prior.p, nullptr, 0,
+                                                                  next_link.p, accepted.p + 4, err.p);
         ::tsr::note_launch();
+        return leaves;
+    };
+    if (pred) {
+        // skip candidates: certify their signs from bounds of their priors
+        DBuf<unsigned long long> ncert(1, st);
+        ncert.zero();
+        DBuf<double2> bnd(nl, st);
+        if (query(need.p, NEED_CERTIFY, bnd.p)) {
+            k_certify<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, esum, ssum, bnd.p, cone_count.p, pred_buf.p, need.p,
+                                                        ncert.p); ::tsr::note_launch();
+            o.certified = read_scalar(ncert.p, st);
+        }
+        // every leaf still needing its prior is queried
+        o.pruned = nl - query(need.p, NEED_QUERY, nullptr);
+    } else {
+        query(nullptr, 0, nullptr);
     }
     o.stage_ms[3] = timer.lap();
     if (update) {
@@ -1200,25 +1489,16 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
         // prior and recompute it, until no such leaf is left (one round
         // queries them all; the next finds none).
         DBuf<uint8_t> mark(nl, st);
-        DBuf<uint32_t> ids(nl, st), flist(nl, st), nsel(1, st);
-        k_iota<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, ids.p); ::tsr::note_launch();
-        size_t tmp = 0;
-        TSR_CUDA(cub::DeviceSelect::Flagged(nullptr, tmp, ids.p, mark.p, flist.p, nsel.p, (int)nl, st));
-        DBuf<uint8_t> tb(tmp, st);
+        DBuf<uint32_t> nmark(1, st);
         for (int round = 0; round < 64; ++round) {
             mark.zero();
+            nmark.zero();
             k_repair_mark<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, t.nb_off.p, t.nbs.p, o.occ.p, need.p, pred, esum, ssum,
                                                             p.confidence_threshold, mark.p); ::tsr::note_launch();
-            TSR_CUDA(cub::DeviceSelect::Flagged(tb.p, tmp, ids.p, mark.p, flist.p, nsel.p, (int)nl, st));
-            const uint32_t nf = read_scalar(nsel.p, st);
+            k_set_needed<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, mark.p, need.p, nmark.p); ::tsr::note_launch();
+            const uint32_t nf = read_scalar(nmark.p, st);
             if (nf == 0) break;
-            k_set_needed<<<grid_for(nf, BLK), BLK, 0, st>>>(nf, flist.p, need.p); ::tsr::note_launch();
-            DBuf<uint32_t> fq = depth_ordered(nf, flist.p, t.leaf_node.p, t.depth.p, st);
-            next_link.zero();
-            k_priors_x<false><<<prior_grid, PT_BLOCK, 0, st>>>(nf, nn, fq.p, t.leaf_node.p, t.leaf_min.p,
-                                                              t.depth.p, t.nmin.p, recs.p, psum.p, t.root_size,
-                                                              p.relative_radius_for_priors, o.prior.p, next_link.p,
-                                                              accepted.p + 4, err.p, nullptr, 0); ::tsr::note_launch();
+            query(mark.p, 1, nullptr);
             k_finalize<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, esum, ssum, elen, slen, o.prior.p, o.cone_count,
                                                          p.confidence_threshold, pred, need.p, o.e_sum.p, o.s_sum.p,
                                                          o.e_len.p, o.s_len.p, o.occ.p); ::tsr::note_launch();
