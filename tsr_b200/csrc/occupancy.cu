@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "handles.h"
@@ -65,35 +66,60 @@ struct TreeIn {
 // te = dot(x - end, m) / denom (= tComplete - 1) and r2 = |x - PCD centre|^2:
 // the confidence-scaled kernel value, or 0 where addKernel adds nothing.
 // Straight-line code (no early exits), so that the lanes of a warp testing
-// different children stay together.
+// different children stay together.  Which products are fused is written out
+// here and below, since it is part of the result: the sums do not change with
+// the code around it.
 __device__ __forceinline__ float kernel_value(const ConeF &c, float te, float r2, bool sampleness, float conf) {
-    const float tcut_m1 = te * c.a_over_l;         // tCut - 1
-    const float tcut = 1.0f + tcut_m1;
-    const float pr = c.radius * (1.0f + te);       // PCD radius at tComplete
-    const float pr2 = pr * pr;
+    const float tcut_m1 = __fmul_rn(te, c.a_over_l);                 // tCut - 1
+    const float tcut = __fmaf_rn(te, c.a_over_l, 1.0f);
+    const float pr = __fmul_rn(c.radius, __fadd_rn(1.0f, te));       // PCD radius at tComplete
+    const float pr2 = __fmul_rn(pr, pr);
     bool ok = (tcut >= 0.0f) & (tcut < 1.0f) & (r2 < pr2);
     float f;   // ray factor: 3/(2Z)(1 - (z/Z)^2) with the 3/(2 L) part in ray_k
     if (sampleness) {
-        const float tcen = fabsf(tcut - 0.5f) * 2.0f;
-        f = 1.0f - tcen * tcen;
+        const float tcen = __fmul_rn(fabsf(__fadd_rn(tcut, -0.5f)), 2.0f);
+        f = __fmaf_rn(-tcen, tcen, 1.0f);
         ok &= tcen < 1.0f;
     } else {
-        f = (-tcut_m1) * (1.0f + tcut);            // (1 - tCut)(1 + tCut)
+        f = __fmul_rn(-tcut_m1, __fadd_rn(1.0f, tcut));              // (1 - tCut)(1 + tCut)
     }
     const float inv = __frcp_rn(pr2);
-    const float kv = c.ray_k * f * (0.63661977236758134f * inv) * (1.0f - r2 * inv);
-    const float scaled = conf * kv;
+    const float kv = __fmul_rn(__fmul_rn(__fmul_rn(c.ray_k, f), __fmul_rn(0.63661977236758134f, inv)),
+                               __fmaf_rn(-r2, inv, 1.0f));
+    const float scaled = __fmul_rn(conf, kv);
     ok &= (kv >= (float)EPS) & (scaled >= (float)EPS);
     return ok ? scaled : 0.0f;
+}
+
+// The offset q of u = x - end from the axis point of the same te, and |q|^2.
+__device__ __forceinline__ void axis_offset(const ConeF &c, F3 u, float te, F3 &q, float &r2) {
+    q = f3(__fmaf_rn(-c.axis.x, te, u.x), __fmaf_rn(-c.axis.y, te, u.y), __fmaf_rn(-c.axis.z, te, u.z));
+    r2 = __fmaf_rn(q.z, q.z, __fmaf_rn(q.x, q.x, __fmul_rn(q.y, q.y)));
 }
 
 // Cone-frame coordinates of point x: te, the offset q from the axis point of
 // the same te, and |q|^2.
 __device__ __forceinline__ void cone_coords(const ConeF &c, F3 x, float &te, F3 &q, float &r2) {
-    F3 u = x - c.end;
-    te = fdot(u, c.m) * c.inv_denom;
-    q = u - c.axis * te;
-    r2 = fdot(q, q);
+    const F3 u = x - c.end;
+    te = __fmul_rn(__fmaf_rn(u.z, c.m.z, __fmaf_rn(u.x, c.m.x, __fmul_rn(u.y, c.m.y))), c.inv_denom);
+    axis_offset(c, u, te, q, r2);
+}
+
+// The same for the centre of child ci of a traversed node.  Its te is rounded
+// as it always was: unfused products in the SAMPLENESS pass, and in the
+// EMPTINESS pass a fused last product for the first five children only.
+template <int TYPE>
+__device__ __forceinline__ void child_coords_of(const ConeF &c, uint32_t ci, F3 x, float &te, F3 &q, float &r2) {
+    const F3 u = x - c.end;
+    float dot;
+    if (TYPE == SAMPLENESS) {
+        dot = __fadd_rn(__fadd_rn(__fmul_rn(u.x, c.m.x), __fmul_rn(u.y, c.m.y)), __fmul_rn(u.z, c.m.z));
+    } else {
+        const float xy = __fmaf_rn(u.x, c.m.x, __fmul_rn(u.y, c.m.y));
+        dot = ci < 5 ? __fmaf_rn(u.z, c.m.z, xy) : __fadd_rn(xy, __fmul_rn(u.z, c.m.z));
+    }
+    te = __fmul_rn(dot, c.inv_denom);
+    axis_offset(c, u, te, q, r2);
 }
 
 __device__ inline float eval_kernel(const ConeF &c, F3 x, bool sampleness, float conf) {
@@ -152,38 +178,21 @@ __device__ __forceinline__ bool separated_at(const ConeF &c, float te, F3 q, flo
     return sep;
 }
 
-constexpr int PT_BLOCK = 128;
-// Resident blocks per SM the persistent traversals are compiled for (the
-// register budget: 65536 / (128 threads x blocks)).
-#ifndef TSR_CONE_E_BLOCKS
-#define TSR_CONE_E_BLOCKS 6
-#endif
-#ifndef TSR_CONE_S_BLOCKS
-#define TSR_CONE_S_BLOCKS 5
+// Resident blocks per SM the traversals are compiled for (the register
+// budget: 65536 / (128 threads x blocks)).
+#ifndef TSR_CONE_BLOCKS
+#define TSR_CONE_BLOCKS 8
 #endif
 #ifndef TSR_PRIOR_BLOCKS
 #define TSR_PRIOR_BLOCKS 4
 #endif
 
-// ------------------------------------------- block-expansion cone traversal
-// Thread-per-link depth-first traversal (the per-link LeavesIterator with a
-// ConeNodesChecker) run by persistent threads: a lane whose traversal ends
-// takes the next link, fetched per warp in one atomic batch, so lanes do not
-// idle behind the warp's longest link.  Child boxes are derived from the
-// parent's box in the link's FP32 frame.  The traversal is organised around
-// children blocks: every step expands one node, loading its eight children's records in one 64-byte
-// line and testing all eight at once, then descends straight into the first
-// surviving child; only nodes with further surviving children go on the
-// stack.  One dependent load per expanded node replaces one per visited
-// child.  Leaf flags are not written here: a leaf got a kernel exactly when
-// its sum is non-zero (every accepted value is >= EPSILON), so they are set
-// afterwards from the sums.
-//
 // Node records: rec[i + 7] = (first child or INVALID, leaf index, with the
 // node's SAMPLENESS flag in bit 31).  Children blocks start at 1 + 8k (root 0,
 // then whole blocks of 8), so a block's records start on a 64-byte boundary.
 // An inner node's second word holds REC_INNER with two bits of what its
-// children block has: flagged leaves, flagged inner nodes.
+// children block has: leaves and inner nodes (flagged ones, once there are
+// flags).
 constexpr uint32_t REC_FLAG = 0x80000000u, REC_NOLEAF = 0x7FFFFFFFu;
 constexpr uint32_t REC_INNER = 0x7FFFFFFCu, REC_HAS_LEAVES = 1u, REC_HAS_INNER = 2u;
 constexpr uint32_t REC_OFFSET = 7;
@@ -194,12 +203,11 @@ __global__ void k_pack_rec(uint32_t nn, const uint32_t *children, const uint32_t
     if (i >= nn) return;
     uint32_t c = children[i];
     uint32_t y = (c == INVALID) ? node_to_leaf[i] : REC_INNER;
-    if (states) {
-        if (states[i] & FLAG_SAMPLENESS) y |= REC_FLAG;
-        if (c != INVALID)
-            for (uint32_t k = 0; k < 8; ++k)
-                if (states[c + k] & FLAG_SAMPLENESS) y |= children[c + k] == INVALID ? REC_HAS_LEAVES : REC_HAS_INNER;
-    }
+    if (states && (states[i] & FLAG_SAMPLENESS)) y |= REC_FLAG;
+    if (c != INVALID)
+        for (uint32_t k = 0; k < 8; ++k)
+            if (!states || (states[c + k] & FLAG_SAMPLENESS))
+                y |= children[c + k] == INVALID ? REC_HAS_LEAVES : REC_HAS_INNER;
     rec[i + REC_OFFSET] = make_uint2(c, y);
 }
 
@@ -263,11 +271,6 @@ __global__ void k_certify(uint32_t nl, const double *esum, const double *ssum, c
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(certified, (unsigned long long)__popc(m));
 }
 
-__device__ __forceinline__ F3 child_min(F3 pmin, uint32_t ci, float size) {
-    return f3((ci & 1u) ? pmin.x + size : pmin.x, (ci & 2u) ? pmin.y + size : pmin.y,
-              (ci & 4u) ? pmin.z + size : pmin.z);
-}
-
 // Per-link set-up of the traversal, precomputed by one thread per link so
 // that the persistent traversal below never runs this long FP64 stretch for a
 // few lanes of a warp while the others wait.  c0 == INVALID: nothing to
@@ -281,23 +284,10 @@ struct __align__(16) LinkRec {
     uint32_t c0;              // children block of the start node
     uint32_t depths;          // depth of those children | max depth << 8
     double spos[3];           // the sample: origin of the FP32 frame
-    uint64_t pad;
+    uint32_t has;             // what the children block has (REC_HAS_LEAVES, REC_HAS_INNER)
+    uint32_t pad;
 };
-
-__device__ __forceinline__ ConeF cone_of(const LinkRec &r) {
-    ConeF c;
-    c.end = f3(r.end[0], r.end[1], r.end[2]);
-    c.axis = f3(r.axis[0], r.axis[1], r.axis[2]);
-    c.m = f3(r.m[0], r.m[1], r.m[2]);
-    c.radius = r.radius;
-    c.full = r.full;
-    c.ray_k = r.ray_k;
-    c.inv_denom = r.inv_denom;
-    c.a_over_l = r.a_over_l;
-    c.t_start_e = r.t_start_e;
-    c.n1 = r.n1;
-    return c;
-}
+static_assert(sizeof(LinkRec) == 128, "copied as eight 16-byte words");
 
 // Set-up of link order[i] (Occupancy.cpp:174-201), FP64, and the start of its
 // traversal: the deepest node containing the cut cone's bounding box.
@@ -409,6 +399,7 @@ __global__ void __launch_bounds__(128) k_link_setup(uint64_t nlinks, const uint3
             r.c0 = srec.x;
             r.depths = (base + 1) | (max_depth << 8);
             r.spos[0] = p.x; r.spos[1] = p.y; r.spos[2] = p.z;
+            r.has = srec.y & (REC_HAS_LEAVES | REC_HAS_INNER);
             r.pad = 0;
         } while (0);
         out[i] = r;
@@ -425,134 +416,212 @@ __global__ void __launch_bounds__(128) k_link_setup(uint64_t nlinks, const uint3
     }
 }
 
-template <int TYPE>
-__global__ void __launch_bounds__(PT_BLOCK, (TYPE == 0) ? TSR_CONE_E_BLOCKS : TSR_CONE_S_BLOCKS) k_cone_x(uint64_t nlinks, const LinkRec *links,
-                                                                         TreeIn tr, const uint2 *rec,
-                                                                         float root_size_f, double *ksum,
-                                                                         double *clen, unsigned long long *accepted,
-                                                                         unsigned long long *next_link,
-                                                                         unsigned long long *visits, int *err,
-                                                                         double sign) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31;
-    // stack of expanded nodes that still have children to descend into
-    uint64_t st[MAX_TREE_DEPTH];   // children block | mask << 32 | depth << 40
-    int sp = 0;
-    D3 spos{0.0, 0.0, 0.0};        // the link's sample: origin of the FP32 frame
-    // the node to expand next: its children block, box corner and depth
-    bool have = false;
-    uint32_t x_c0 = 0, x_d = 0;
-    F3 x_min = f3(0.f, 0.f, 0.f);
-    uint32_t max_depth = 0;
-    ConeF c;
-    double wlen = 0.0;
-    float fconf = 0.f;
-    bool done = false;
-    unsigned long long acc = 0, nvis = 0;
+// ------------------------------------------- cone traversal
+// The links' depth-first traversals (the per-link LeavesIterator with a
+// ConeNodesChecker), a warp taking CX_LINKS links at a time.  The blocks of
+// children to visit lie on one stack per warp, whichever link they belong to,
+// and a step takes four of them, one child a lane: every lane works whatever
+// the links' lengths, and one long link is shared by all lanes.  (A lane per
+// link left 8 of 32 lanes busy at 300k samples and 21 at 16M, and ended on the
+// longest link.)  The links' cones lie in shared memory.  As in the prior
+// queries there are two kinds of steps: inner nodes get the box test, and
+// their children blocks go on the stack; leaves get the kernel.
+//
+// Measured, SAMPLENESS + EMPTINESS pass: 14 + 24 -> 2.3 + 5.3 ms at 300k
+// held-out samples, 20 + 30 -> 15 + 27 ms at 4M CSG, 99 + 247 -> 59 + 190 ms
+// at 16M held-out.  What bounds it is instruction issue (3.2 of 4 a clock); the
+// FP64 atomics keep their L2 units 8 % busy.
+//
+// The FP32 arithmetic of a child's box is part of the result, so it follows
+// one rule: the first surviving child's corner comes from its parent's by the
+// FP32 recurrence, every other one's from the FP64 tree.
+//
+// Leaf flags are not written here: a leaf got a kernel exactly when its sum is
+// non-zero (every accepted value is >= EPSILON), so they are set afterwards
+// from the sums.
+constexpr int CX_LINKS = 8;
+constexpr int CX_WIDE = 96;     // from here on a step takes one block, which adds at most 7 a level
+constexpr int CX_LEAVES = 64;   // blocks whose leaves wait; worked off when fewer than 32 are free
+constexpr int CX_WARPS = 4;
 
+// A warp's stack entries for a tree of that depth: a wide step leaves at most
+// CX_WIDE + 28, a narrow one adds 7 a level.
+inline uint32_t cone_stack(uint32_t tree_depth) { return (CX_WIDE + 28 + 7 * tree_depth + 8 + 7) & ~7u; }
+
+struct ConeWarp {
+    float4 link[CX_LINKS][9];       // LinkRec; the ninth word keeps four links' words in different banks
+    float4 leaf_box[CX_LEAVES];     // a block's corner (the link's frame) and index
+    uint16_t leaf_tag[CX_LEAVES];   // its link's place, and its nodes' depth << 3
+    float4 box[1];                  // the stack, of the tree's depth; its tags follow
+};
+
+inline size_t cone_warp_bytes(uint32_t stack) {
+    return (offsetof(ConeWarp, box) + stack * (sizeof(float4) + sizeof(uint16_t)) + 15) & ~(size_t)15;
+}
+
+__device__ __forceinline__ ConeF cone_of(const float4 *l) {
+    const float4 a = l[0], b = l[1], c = l[2], d = l[3];
+    ConeF k;
+    k.end = f3(a.x, a.y, a.z);
+    k.axis = f3(a.w, b.x, b.y);
+    k.m = f3(b.z, b.w, c.x);
+    k.radius = c.y;
+    k.full = c.z;
+    k.ray_k = c.w;
+    k.inv_denom = d.x;
+    k.a_over_l = d.y;
+    k.t_start_e = d.z;
+    k.n1 = d.w;
+    return k;
+}
+
+template <int TYPE>
+__global__ void __launch_bounds__(32 * CX_WARPS, TSR_CONE_BLOCKS)
+    k_cones(uint64_t nlinks, uint32_t per, uint32_t stack, uint32_t warp_bytes, const LinkRec *links, TreeIn tr, const uint2 *rec, float root_size_f,
+            double *ksum, double *clen, unsigned long long *accepted, unsigned long long *next_link,
+            unsigned long long *visits, int *err, double sign) {
+    const unsigned FULL = 0xffffffffu;
+    extern __shared__ float4 cone_shared[];
+    __shared__ float sizes[64];     // edge length of a node at a depth
+    ConeWarp &w = *reinterpret_cast<ConeWarp *>(reinterpret_cast<char *>(cone_shared) + (threadIdx.x >> 5) * warp_bytes);
+    float4 *const stack_box = w.box;
+    uint16_t *const stack_tag = reinterpret_cast<uint16_t *>(w.box + stack);
+    const unsigned lane = threadIdx.x & 31, below = (1u << lane) - 1u, ci = lane & 7u;
+    const int quarter = (int)(lane >> 3);
+    const float bx = (float)(ci & 1u), by = (float)((ci >> 1) & 1u), bz = (float)(ci >> 2), fsign = (float)sign;
+    if (threadIdx.x < 64) sizes[threadIdx.x] = ldexpf(root_size_f, -(int)threadIdx.x);
+    __syncthreads();
+    uint32_t hits = 0, expanded = 0;   // of this lane, since the last links
+    unsigned long long acc = 0, nvis = 0;
+    int sp = 0, waiting = 0;
     while (true) {
-        // resume the deepest expanded node that has children left
-        if (!have && sp > 0) {
-            uint64_t e = st[sp - 1];
-            uint32_t m = (uint32_t)(e >> 32) & 0xFFu;
-            uint32_t node = (uint32_t)e + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1;
-            if (m) st[sp - 1] = (e & ~(0xFFull << 32)) | ((uint64_t)m << 32); else --sp;
-            x_c0 = __ldg(&rec[node + REC_OFFSET]).x;
-            x_min = rel(tr.nmin[node], spos);
-            x_d = (uint32_t)(e >> 40) + 1;
-            have = true;
-        }
-        bool need = !have && !done;
-        unsigned nm = __ballot_sync(FULL, need);
-        if (nm) {
-            int leader = __ffs(nm) - 1;
-            unsigned long long b = 0;
-            if ((int)lane == leader) b = atomicAdd(next_link, (unsigned long long)__popc(nm));
-            b = __shfl_sync(FULL, b, leader);
-            if (need) {
-                uint64_t i = b + __popc(nm & ((1u << lane) - 1u));
-                if (i >= nlinks) {
-                    done = true;
-                } else {
-                    const LinkRec r = links[i];
-                    if (r.c0 != INVALID) {
-                        c = cone_of(r);
-                        wlen = r.wlen;
-                        fconf = r.fconf;
-                        max_depth = r.depths >> 8;
-                        spos = D3{r.spos[0], r.spos[1], r.spos[2]};
-                        x_c0 = r.c0;
-                        x_min = f3(r.smin[0], r.smin[1], r.smin[2]);
-                        x_d = r.depths & 0xFFu;
-                        have = true;
-                    }
+        if (sp == 0 && waiting == 0) {
+            acc += hits;
+            nvis += 8ull * expanded;
+            hits = expanded = 0;
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(next_link, (unsigned long long)per);
+            base = __shfl_sync(FULL, base, 0);
+            if (base >= nlinks) break;
+            const uint32_t n = (uint32_t)min((unsigned long long)per, nlinks - base);
+            const float4 *src = reinterpret_cast<const float4 *>(links + base);
+            for (uint32_t i = lane; i < 8 * n; i += 32) w.link[i >> 3][i & 7] = __ldg(src + i);
+            __syncwarp();
+            bool start = false;
+            uint32_t has = 0;
+            float4 box = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint16_t tag = 0;
+            if (lane < n) {
+                const LinkRec &r = *reinterpret_cast<const LinkRec *>(w.link[lane]);
+                if (r.c0 != INVALID) {
+                    start = true;
+                    has = r.has;
+                    box = make_float4(r.smin[0], r.smin[1], r.smin[2], __uint_as_float((r.c0 - 1) >> 3));
+                    tag = (uint16_t)(lane | ((r.depths & 0xFFu) << 3));
                 }
             }
-        }
-        if (__all_sync(FULL, done && !have && sp == 0)) break;
-        if (!have) continue;
-        // ---- expand: test the eight children of the node (NodesIterator.cpp:38-86)
-        have = false;
-        if ((x_c0 & 7u) != 1u || x_c0 > 0xFFFFFFF0u) {   // children blocks start at 1 + 8k
-            atomicExch(err, 3);
+            const bool push = start && (has & REC_HAS_INNER), wait = start && (has & REC_HAS_LEAVES);
+            const unsigned pm = __ballot_sync(FULL, push), wm = __ballot_sync(FULL, wait);
+            if (push) {
+                const int j = __popc(pm & below);
+                stack_box[j] = box;
+                stack_tag[j] = tag;
+            }
+            if (wait) {
+                const int j = __popc(wm & below);
+                w.leaf_box[j] = box;
+                w.leaf_tag[j] = tag;
+            }
+            sp = __popc(pm);
+            waiting = __popc(wm);
+            expanded += start;
+            __syncwarp();
             continue;
         }
-        const uint4 *line = reinterpret_cast<const uint4 *>(rec + x_c0 + REC_OFFSET);
-        uint4 q0 = __ldg(line), q1 = __ldg(line + 1), q2 = __ldg(line + 2), q3 = __ldg(line + 3);
-        const uint32_t rx[8] = {q0.x, q0.z, q1.x, q1.z, q2.x, q2.z, q3.x, q3.z};
-        const uint32_t ry[8] = {q0.y, q0.w, q1.y, q1.w, q2.y, q2.w, q3.y, q3.w};
-        const float size = ldexpf(root_size_f, -(int)x_d);
-        const bool can_descend = x_d + 1 <= max_depth;
+        if (waiting > CX_LEAVES - 32 || sp == 0) {
+            // ---- the leaves of the waiting blocks: addKernel's exact test decides, no box test needed
+            do {
+                const bool valid = quarter < waiting;
+                const int at = valid ? waiting - 1 - quarter : 0;
+                const float4 b = w.leaf_box[at];
+                const uint32_t tag = w.leaf_tag[at];
+                const uint2 r = __ldg(&rec[1 + 8 * __float_as_uint(b.w) + ci + REC_OFFSET]);
+                const float4 *l = w.link[tag & 7u];
+                const ConeF c = cone_of(l);
+                const float size = sizes[tag >> 3], h = 0.5f * size;
+                const F3 ctr0 = f3(b.x, b.y, b.z) + f3(h, h, h);
+                const F3 ctr = f3(fmaf(bx, size, ctr0.x), fmaf(by, size, ctr0.y), fmaf(bz, size, ctr0.z));
+                float te, r2;
+                F3 q;
+                child_coords_of<TYPE>(c, ci, ctr, te, q, r2);
+                const float val = kernel_value(c, te, r2, TYPE == SAMPLENESS, l[4].w);
+                const bool hit = valid && r.x == INVALID && (TYPE == SAMPLENESS || (r.y & REC_FLAG)) && val > 0.0f;
+                if (hit) {
+                    const uint32_t lf = r.y & REC_NOLEAF;
+                    const double wlen = *reinterpret_cast<const double *>(l + 5);   // carries the sign
+                    atomicAdd(&ksum[lf], (double)(fsign * val));
+                    atomicAdd(&clen[lf], wlen);
+                    ++hits;
+                }
+                waiting -= 4;
+            } while (waiting >= 4 || (waiting > 0 && sp == 0));
+            if (waiting < 0) waiting = 0;
+            __syncwarp();
+            continue;
+        }
+        // ---- the inner nodes of the blocks on top of the stack
+        const int take = sp > CX_WIDE ? 1 : (sp < 4 ? sp : 4);
+        const bool valid = quarter < take;
+        const int at = sp - 1 - (valid ? quarter : 0);
+        const float4 b = stack_box[at];
+        const uint32_t tag = stack_tag[at], d = tag >> 3;
+        sp -= take;
+        const uint32_t node = 1 + 8 * __float_as_uint(b.w) + ci;
+        const uint2 r = __ldg(&rec[node + REC_OFFSET]);
+        const LinkRec *l = reinterpret_cast<const LinkRec *>(w.link[tag & 7u]);
+        const ConeF c = cone_of(w.link[tag & 7u]);
+        const float size = sizes[d], h = 0.5f * size;
+        const F3 x_min = f3(b.x, b.y, b.z), ctr0 = x_min + f3(h, h, h);
         // one widened half size for all eight boxes: covers the FP32 corner
         // error of every child centre (|centre|_1 <= |x_min|_1 + 4.5 size)
-        const float h = 0.5f * size;
         const float hs = h + 2e-6f * (fabsf(x_min.x) + fabsf(x_min.y) + fabsf(x_min.z) + 4.5f * size);
         const float dt = hs * c.n1 * fabsf(c.inv_denom);
-        const F3 ctr0 = x_min + f3(h, h, h);
-        uint32_t mask = 0;
-        nvis += 8;
-#pragma unroll
-        for (int ci = 0; ci < 8; ++ci) {
-            // both tests for every child, without branches; only the outcome
-            // (a leaf's kernel, or a child to descend into) is conditional
-            const bool flagged = TYPE == SAMPLENESS || (ry[ci] & REC_FLAG);
-            const bool leaf = rx[ci] == INVALID;
-            F3 ctr = f3((ci & 1) ? ctr0.x + size : ctr0.x, (ci & 2) ? ctr0.y + size : ctr0.y,
-                        (ci & 4) ? ctr0.z + size : ctr0.z);
-            float te, r2;
-            F3 q;
-            cone_coords(c, ctr, te, q, r2);
-            const float val = kernel_value(c, te, r2, TYPE == SAMPLENESS, fconf);
-            const bool sep = separated_at(c, te, q, r2, hs, dt);
-            // a leaf: addKernel's exact test decides, no box test needed
-            if (flagged && leaf && val > 0.0f) {
-                uint32_t lf = ry[ci] & REC_NOLEAF;
-                atomicAdd(&ksum[lf], sign * (double)val);
-                atomicAdd(&clen[lf], wlen);   // wlen carries the sign
-                ++acc;
-            }
-            if (flagged && !leaf && can_descend && !sep) mask |= 1u << ci;
+        const F3 ctr = f3(fmaf(bx, size, ctr0.x), fmaf(by, size, ctr0.y), fmaf(bz, size, ctr0.z));
+        float te, r2;
+        F3 q;
+        child_coords_of<TYPE>(c, ci, ctr, te, q, r2);
+        const bool sep = separated_at(c, te, q, r2, hs, dt);
+        const bool next = valid && r.x != INVALID && (TYPE == SAMPLENESS || (r.y & REC_FLAG)) && !sep &&
+                          d + 1 <= (l->depths >> 8);
+        const unsigned nm = __ballot_sync(FULL, next);
+        float4 box = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (next) {
+            const bool first = ((nm >> (lane & 24u)) & ((1u << ci) - 1u)) == 0;
+            F3 x = f3(fmaf(bx, size, x_min.x), fmaf(by, size, x_min.y), fmaf(bz, size, x_min.z));
+            if (!first) x = rel(tr.nmin[node], D3{l->spos[0], l->spos[1], l->spos[2]});
+            box = make_float4(x.x, x.y, x.z, __uint_as_float((r.x - 1) >> 3));
         }
-        if (mask) {
-            uint32_t ci = __ffs(mask) - 1;
-            uint32_t rest = mask & (mask - 1);
-            if (rest) {
-                if (sp >= MAX_TREE_DEPTH) {
-                    atomicExch(err, 1);
-                    continue;
-                }
-                st[sp++] = (uint64_t)x_c0 | ((uint64_t)rest << 32) | ((uint64_t)x_d << 40);
+        const uint16_t ntag = (uint16_t)(tag + 8);   // one deeper
+        const bool push = next && (r.y & REC_HAS_INNER), wait = next && (r.y & REC_HAS_LEAVES);
+        const unsigned pm = __ballot_sync(FULL, push), wm = __ballot_sync(FULL, wait);
+        if (sp + __popc(pm) > (int)stack) {
+            if (lane == 0) atomicExch(err, 1);
+        } else {
+            if (push) {
+                const int j = sp + __popc(pm & below);
+                stack_box[j] = box;
+                stack_tag[j] = ntag;
             }
-            uint32_t nc = rx[0];
-#pragma unroll
-            for (int k = 1; k < 8; ++k)
-                if (ci == (uint32_t)k) nc = rx[k];
-            x_min = child_min(x_min, ci, size);
-            x_c0 = nc;
-            x_d += 1;
-            have = true;
+            sp += __popc(pm);
         }
+        if (wait) {
+            const int j = waiting + __popc(wm & below);
+            w.leaf_box[j] = box;
+            w.leaf_tag[j] = ntag;
+        }
+        waiting += __popc(wm);
+        expanded += next;
+        __syncwarp();
     }
     for (int o = 16; o; o >>= 1) {
         acc += __shfl_xor_sync(FULL, acc, o);
@@ -1308,18 +1377,23 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
     TreeIn tr{t.nmin.p};
     if (!update) o.links = nlinks;
     DBuf<unsigned long long> next_link(1, st);
+    const uint32_t stack = cone_stack(t.max_depth), warp_bytes = (uint32_t)cone_warp_bytes(stack);
+    const size_t cone_smem = (size_t)CX_WARPS * warp_bytes;
     unsigned x_grid = 0, prior_grid = 0, bounds_grid = 0;
     {
         int dev = 0, sms = 0, per_sm = 0;
         TSR_CUDA(cudaGetDevice(&dev));
         TSR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cone_x<EMPTINESS>, PT_BLOCK, 0));
+        TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cones<EMPTINESS>, 32 * CX_WARPS, cone_smem));
         x_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
         TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_priors<false>, 32 * PP_WARPS, 0));
         prior_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
         TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_priors<true>, 32 * PP_WARPS, 0));
         bounds_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
     }
+    // links a warp takes at a time: so few that every warp gets some
+    const uint32_t links_per_warp =
+        (uint32_t)std::min<uint64_t>(CX_LINKS, std::max<uint64_t>(1, nlinks / ((uint64_t)x_grid * CX_WARPS * 2)));
     if (nl > REC_NOLEAF) fail(TSR_ERR_OVERFLOW_U32, "leaf count must stay below 2^31 - 1 for the traversal records");
     DBuf<uint2> recs((size_t)nn + 8, st);
     if (reinterpret_cast<uintptr_t>(recs.p) % 16) fail(TSR_ERR_CUDA, "traversal records are not 16-byte aligned");
@@ -1331,7 +1405,7 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
                                                                         ssum, slen, cone_count.p, accepted.p + 1,
                                                                         sign);
         ::tsr::note_launch();
-        k_cone_x<SAMPLENESS><<<x_grid, PT_BLOCK, 0, st>>>(nlinks, lrec.p, tr, recs.p, (float)t.root_size, ssum, slen,
+        k_cones<SAMPLENESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, ssum, slen,
                                                          accepted.p + 1, next_link.p, accepted.p + 3, err.p, sign);
         ::tsr::note_launch();
     }
@@ -1375,7 +1449,7 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
         k_link_setup<EMPTINESS><<<grid_for(nlinks, 128), 128, 0, st>>>(nlinks, order.p, in, tr, recs.p, lrec.p, esum,
                                                                        elen, cone_count.p, accepted.p, sign);
         ::tsr::note_launch();
-        k_cone_x<EMPTINESS><<<x_grid, PT_BLOCK, 0, st>>>(nlinks, lrec.p, tr, recs.p, (float)t.root_size, esum, elen,
+        k_cones<EMPTINESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, esum, elen,
                                                         accepted.p, next_link.p, accepted.p + 2, err.p, sign);
         ::tsr::note_launch();
     }
@@ -1515,7 +1589,6 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
     o.visits[0] = a[2];
     o.visits[1] = a[3];
     o.visits[2] = a[4];
-    if (e == 3) fail(TSR_ERR_DEVICE_ASSERT, "occupancy traversal met a children block off its 8-node alignment");
     if (e) fail(TSR_ERR_DEVICE_ASSERT, "occupancy traversal exceeded its stack bound");
     TSR_CUDA(cudaGetLastError());
 }
