@@ -177,32 +177,6 @@ __host__ __device__ inline bool aabb_sphere(const D3 &mn, const D3 &mx, const D3
     return d2 <= dmul(r, r);
 }
 
-// Slab clipping of s + t (e - s), t in [0, 1].
-__host__ __device__ inline bool segment_aabb(double &t0, double &t1, const D3 &s, const D3 &e,
-                                             const D3 &mn, const D3 &mx) {
-    double lo = 0.0, hi = 1.0;
-    const double sv[3] = {s.x, s.y, s.z};
-    const double dv[3] = {dsub(e.x, s.x), dsub(e.y, s.y), dsub(e.z, s.z)};
-    const double bmn[3] = {mn.x, mn.y, mn.z};
-    const double bmx[3] = {mx.x, mx.y, mx.z};
-    for (int a = 0; a < 3; ++a) {
-        if (dv[a] == 0.0) {
-            if (sv[a] < bmn[a] || sv[a] > bmx[a]) return false;
-            continue;
-        }
-        double inv = 1.0 / dv[a];
-        double ta = dmul(dsub(bmn[a], sv[a]), inv);
-        double tb = dmul(dsub(bmx[a], sv[a]), inv);
-        if (ta > tb) { double t = ta; ta = tb; tb = t; }
-        if (ta > lo) lo = ta;
-        if (tb < hi) hi = tb;
-        if (lo > hi) return false;
-    }
-    t0 = lo;
-    t1 = hi;
-    return true;
-}
-
 // Node edge length at a depth: repeated exact halving of the root size.
 __host__ __device__ inline double size_at(double root_size, uint32_t depth) {
     double s = root_size;

@@ -238,69 +238,107 @@ __device__ inline uint32_t sphere_start_v(const NV &v, const Root &root, uint32_
     return node;
 }
 
-// Nodes::findReliableSamplingNode (Nodes.cpp:433-469) over the versioned
-// tree, from `start` (the root, or a node that contains the side's sphere,
-// see sphere_start_v); calls on_read(leaf) for every leaf it rejects.
-// Returns the reliable leaf or INVALID.  The order is the reference's
-// depth-first order (children 0..7, each subtree before the next sibling),
-// which decides the returned leaf.
-template <class OnRead>
-__device__ uint32_t find_reliable_v(const NV &v, const Root &root, uint32_t start, uint32_t key,
-                                    const SampleRef &q, OnRead on_read, int *err) {
-    if (leaf_v(v, start, key)) {
-        D3 smn = start ? v.nmin[start] : root.mn;
-        double ssz = start ? size_at(root.size, v.depth[start]) : root.size;
-        if (leaf_reliable(smn, ssz, q)) return start;
-        on_read(start);
-        return INVALID;
+// A side's tests in FP32, in the frame of its sample, with their error bounds:
+// they decide all but the few boxes within the bounds, which the FP64 tests
+// above decide, at up to a hundred half-rate operations a box.
+enum Decision { NO = 0, YES = 1, UNSURE = 2 };
+
+struct SideF {
+    float nx, ny, nz, n_lo, n_hi, r2;   // normal, its negative and positive parts' sums, r^2
+    float e, e_plane;                   // error bounds: of a corner, and of a plane distance
+    bool positive;
+
+    __device__ __forceinline__ SideF() {}
+    // `reach`: no coordinate of a box of the search exceeds it; `margin`: bound
+    // of the FP64 rounding (see sphere_start_v).  A corner is one rounded
+    // difference and at most MAX_TREE_DEPTH rounded steps; 2^-24 x (40 + 4)
+    // stays below 3e-6.
+    __device__ __forceinline__ SideF(const SampleRef &q, float reach, float margin) {
+        nx = (float)q.n.x;
+        ny = (float)q.n.y;
+        nz = (float)q.n.z;
+        n_lo = fminf(nx, 0.0f) + fminf(ny, 0.0f) + fminf(nz, 0.0f);
+        n_hi = fmaxf(nx, 0.0f) + fmaxf(ny, 0.0f) + fmaxf(nz, 0.0f);
+        const float r = (float)q.r;
+        r2 = r * r;
+        e = 3e-6f * reach + margin;
+        e_plane = 2.0f * (n_hi - n_lo) * e;
+        positive = q.positive;
     }
-    // The node being scanned lives in registers (its children block, corner,
-    // depth and next child); children's corners come from the build's own
-    // recurrence (child_coords, exact), so a child costs a load only when it
-    // meets the side.  Stack entries are (node, next child); resuming reloads
-    // the node's block, corner and depth.
-    uint64_t st[MAX_TREE_DEPTH];
-    int sp = 0;
-    uint32_t cur = start, c0 = v.children[start], next = 0, d = v.depth[start];
-    D3 pmn = start ? v.nmin[start] : root.mn;
-    double cs = size_at(root.size, d + 1);
-    while (true) {
-        if (next == 8) {
-            if (sp == 0) return INVALID;
-            uint64_t e = st[--sp];
-            cur = (uint32_t)e;
-            next = (uint32_t)(e >> 32);
-            c0 = v.children[cur];
-            d = v.depth[cur];
-            pmn = cur ? v.nmin[cur] : root.mn;
-            cs = size_at(root.size, d + 1);
-            continue;
-        }
-        uint32_t c = next++;
-        D3 cmn = child_coords(pmn, cs, c);
-        if (!intersect_side(cmn, cs, q)) continue;
-        uint32_t idx = c0 + c;
-        uint32_t ch = v.children[idx];
-        if (ch == INVALID || v.cc[idx] >= key) {   // leaf_v
-            if (leaf_reliable(cmn, cs, q)) return idx;
-            on_read(idx);
-            continue;
-        }
-        if (next < 8) {   // nothing to resume after the last child
-            if (sp >= MAX_TREE_DEPTH) { *err = 1; return INVALID; }
-            st[sp++] = (uint64_t)cur | ((uint64_t)next << 32);
-        }
-        cur = idx;
-        c0 = ch;
-        pmn = cmn;
-        ++d;
-        cs = dmul(cs, 0.5);
-        next = 0;
+    // d2 against r2, each with its rounding; t = the sum of the terms squared
+    __device__ __forceinline__ Decision within(float d2, float t) const {
+        const float err = 2.0f * e * t + 3.0f * e * e + 1e-6f * (d2 + r2), d = d2 - r2;
+        return d < -err ? YES : (d > err ? NO : UNSURE);
     }
-}
+    // a point at plane distance s lies on the side
+    __device__ __forceinline__ Decision on_side(float s) const {
+        const float d = positive ? s : -s;
+        return d > e_plane ? YES : (d < -e_plane ? NO : UNSURE);
+    }
+    // intersect_side of the box at corner (x, y, z)
+    __device__ __forceinline__ Decision box(float x, float y, float z, float size) const {
+        const float s = fmaf(nz, z, fmaf(ny, y, nx * x));
+        const Decision side = on_side(fmaf(size, positive ? n_hi : n_lo, s));
+        const float tx = fmaxf(fmaxf(x, -(x + size)), 0.0f), ty = fmaxf(fmaxf(y, -(y + size)), 0.0f),
+                    tz = fmaxf(fmaxf(z, -(z + size)), 0.0f);
+        const Decision near = within(fmaf(tz, tz, fmaf(ty, ty, tx * tx)), tx + ty + tz);
+        return side == NO || near == NO ? NO : (side == YES && near == YES ? YES : UNSURE);
+    }
+    // fitting_center of the point (x, y, z)
+    __device__ __forceinline__ Decision center(float x, float y, float z) const {
+        const Decision near = within(fmaf(z, z, fmaf(y, y, x * x)), fabsf(x) + fabsf(y) + fabsf(z));
+        const Decision side = on_side(fmaf(nz, z, fmaf(ny, y, nx * x)));
+        return side == NO || near == NO ? NO : (side == YES && near == YES ? YES : UNSURE);
+    }
+    // leaf_reliable of the leaf at corner (x, y, z)
+    __device__ __forceinline__ Decision reliable(float x, float y, float z, float size) const {
+        const float cs = 0.5f * size, g = 0.25f * size;
+        const Decision c = center(x + cs, y + cs, z + cs);
+        if (c != YES) return c;
+        bool unsure = false;
+#pragma unroll 2
+        for (uint32_t i = 0; i < 8; ++i) {
+            const Decision k = center(((i & 1u) ? x + cs : x) + g, ((i & 2u) ? y + cs : y) + g, ((i & 4u) ? z + cs : z) + g);
+            if (k == YES) return YES;
+            unsure |= k == UNSURE;
+        }
+        return unsure ? UNSURE : NO;
+    }
+};
+
+// Slab clipping of s + t (e - s), t in [0, 1], with the segment's reciprocals
+// taken once for all boxes.
+struct Segment {
+    double s[3], d[3], inv[3];
+    __device__ inline Segment(const D3 &a, const D3 &e) {
+        s[0] = a.x; s[1] = a.y; s[2] = a.z;
+        d[0] = dsub(e.x, a.x); d[1] = dsub(e.y, a.y); d[2] = dsub(e.z, a.z);
+        for (int k = 0; k < 3; ++k) inv[k] = 1.0 / d[k];
+    }
+    __device__ inline bool clip(double &t0, double &t1, const D3 &mn, const D3 &mx) const {
+        double lo = 0.0, hi = 1.0;
+        const double bmn[3] = {mn.x, mn.y, mn.z}, bmx[3] = {mx.x, mx.y, mx.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (d[a] == 0.0) {
+                if (s[a] < bmn[a] || s[a] > bmx[a]) return false;
+                continue;
+            }
+            double ta = dmul(dsub(bmn[a], s[a]), inv[a]);
+            double tb = dmul(dsub(bmx[a], s[a]), inv[a]);
+            if (ta > tb) { double t = ta; ta = tb; tb = t; }
+            if (ta > lo) lo = ta;
+            if (tb < hi) hi = tb;
+            if (lo > hi) return false;
+        }
+        t0 = lo;
+        t1 = hi;
+        return true;
+    }
+};
 
 // Child with the largest overlap with the sampling segment (Nodes.cpp:300-331).
-__device__ inline uint32_t best_child(const D3 &mn, double size, const D3 &p, const D3 &endp) {
+__device__ inline uint32_t best_child(const D3 &mn, double size, const Segment &seg) {
     double cs = dmul(size, 0.5);
     double score = -REAL_MAX;
     uint32_t best = INVALID;
@@ -308,7 +346,7 @@ __device__ inline uint32_t best_child(const D3 &mn, double size, const D3 &p, co
         D3 bmin = child_coords(mn, cs, c);
         D3 bmax{dadd(bmin.x, cs), dadd(bmin.y, cs), dadd(bmin.z, cs)};
         double t0, t1;
-        if (!segment_aabb(t0, t1, p, endp, bmin, bmax)) continue;
+        if (!seg.clip(t0, t1, bmin, bmax)) continue;
         double ov = dsub(t1, t0);
         if (ov <= score) continue;
         score = ov;
@@ -327,12 +365,12 @@ __device__ inline D3 segment_end(const SampleRef &q) {
 // (started at a node that contains the side's sphere, see sphere_start_v).
 __device__ inline uint32_t descent_leaf_v(const NV &v, const Root &root, uint32_t start, uint32_t key,
                                           const SampleRef &q, int *err) {
-    D3 endp = segment_end(q);
+    const Segment seg(q.p, segment_end(q));
     uint32_t node = start;
     for (int guard = 0; guard < 4 * MAX_TREE_DEPTH; ++guard) {
         if (leaf_v(v, node, key)) return node;
         double sz = size_at(root.size, v.depth[node]);
-        uint32_t b = best_child(v.nmin[node], sz, q.p, endp);
+        uint32_t b = best_child(v.nmin[node], sz, seg);
         if (b == INVALID) { *err = 2; return node; }
         node = v.children[node] + b;
     }
@@ -340,32 +378,199 @@ __device__ inline uint32_t descent_leaf_v(const NV &v, const Root &root, uint32_
     return node;
 }
 
-// Round evaluation: status 1 = reliable (witness), 2 = writer.  Also counts
-// each side's dependency pairs (1 for a witness; the rejected leaves plus the
-// descent leaf for a writer).
-// split_sides: the keys are both sides of consecutive samples in turn (the
-// first round); threads then take all positive sides first and all negative
-// sides after them, so the lanes of a warp search in the same direction
-// (the two sides' searches differ, and a warp waits for its longest one).
-// Results go to each side's own slot either way.
-__global__ void k_sampling_eval(uint32_t m, const uint32_t *keys, NV v, Root root, const D3 *pos, const D3 *nrm,
-                                const double *scale, double h_svo, uint8_t *status, uint32_t *witness,
-                                uint32_t *dleaf, uint32_t *cnt, double margin, int *err, int split_sides) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    const uint32_t half = (m + 1) / 2;
-    const uint32_t i = split_sides ? (t < half ? 2 * t : 2 * (t - half) + 1) : t;
-    uint32_t key = keys[i];
-    SampleRef q = sample_side(key, pos, nrm, scale, h_svo);
+// Where every side's search starts and the leaf its best-overlap descent reaches.
+__global__ void __launch_bounds__(128) k_sides_begin(uint32_t m, const uint32_t *keys, NV v, Root root, const D3 *pos,
+                                                    const D3 *nrm, const double *scale, double h_svo, uint32_t *start,
+                                                    uint32_t *dleaf, double margin, int *err) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t key = keys[i];
+    const SampleRef q = sample_side(key, pos, nrm, scale, h_svo);
     int e = 0;
-    uint32_t reads = 0;
-    uint32_t start = sphere_start_v(v, root, key, q, margin);
-    uint32_t w = find_reliable_v(v, root, start, key, q, [&](uint32_t) { ++reads; }, &e);
-    status[i] = (w != INVALID) ? 1 : 2;
-    witness[i] = w;
-    cnt[i] = (w != INVALID) ? 1u : reads + 1u;
-    dleaf[i] = descent_leaf_v(v, root, start, key, q, &e);
+    const uint32_t at = sphere_start_v(v, root, key, q, margin);
+    start[i] = at;
+    dleaf[i] = descent_leaf_v(v, root, at, key, q, &e);
     if (e) atomicExch(err, e);
+}
+
+// Nodes::findReliableSamplingNode (Nodes.cpp:433-469) over the versioned tree
+// for every side, from its start (the root, or a node that contains the
+// side's sphere, see sphere_start_v): the first reliable leaf in the
+// reference's depth-first order (children 0..7, each subtree before the next
+// sibling), or none after all leaves that meet the side were rejected.
+//
+// Eight lanes search for one side: a step tests a node's eight children, one
+// a lane, boxes and leaves alike; the lowest child that is a reliable leaf or
+// an inner node decides what is next, and the higher ones go on the group's
+// stack in shared memory.  The groups take sides from a counter.  A thread per
+// side in FP64 kept 5 of 32 lanes busy, since searches differ in length, and
+// its chain of dependent loads was eight times as long: both searches and the
+// descents took 67 ms at 16M held-out samples and 21 ms at 4M CSG, and take 54
+// and 15 now, 19 lanes busy; a round's resolution, with the writers' second
+// search, 14 -> 12 ms at 4M.  What bounds it is issue and the load of each
+// node's children.
+//
+// Round evaluation (LIST false): status 1 = reliable (the witness), 2 = writer,
+// and each side's number of dependency pairs: 1 for a witness, the rejected
+// leaves plus the descent leaf for a writer.
+//
+// Dependency lists of the writers (LIST true; `sides` are the writers): the
+// leaves the search rejected, as (leaf, side) pairs from off[side] on.
+template <bool LIST>
+__global__ void __launch_bounds__(128) k_search(uint32_t m, const uint32_t *sides, const uint32_t *keys, NV v,
+                                               Root root, const D3 *pos, const D3 *nrm, const double *scale,
+                                               double h_svo, const uint32_t *start, uint8_t *status,
+                                               uint32_t *witness, uint32_t *cnt, const uint32_t *off, uint32_t *skeys,
+                                               uint32_t *svals, double margin, uint32_t *next_side, int *err) {
+    const unsigned FULL = 0xffffffffu;
+    __shared__ uint64_t stacks[16][MAX_TREE_DEPTH];   // block | children left << 32 | reliable ones << 40 | depth << 48
+    __shared__ double sizes[MAX_TREE_DEPTH + 8];      // edge length at a depth
+    uint64_t *st = stacks[threadIdx.x >> 3];
+    const unsigned lane = threadIdx.x & 31, ci = lane & 7u, shift = lane & 24u;
+    if (threadIdx.x < MAX_TREE_DEPTH + 8) sizes[threadIdx.x] = size_at(root.size, threadIdx.x);
+    __syncthreads();
+    bool have = false, done = false;
+    uint32_t i = 0, key = 0, c0 = 0, d = 0, reads = 0;   // d: depth of the children of block c0
+    int sp = 0;
+    float px = 0.f, py = 0.f, pz = 0.f;
+    SampleRef q{};
+    SideF f;
+    while (true) {
+        const unsigned want = __ballot_sync(FULL, !have && !done && ci == 0);
+        if (want) {
+            uint32_t base = 0;
+            const int leader = __ffs(want) - 1;
+            if ((int)lane == leader) base = atomicAdd(next_side, (uint32_t)__popc(want));
+            base = __shfl_sync(FULL, base, leader);
+            if (!have && !done) {
+                const uint32_t j = base + __popc(want & ((1u << shift) - 1u));
+                if (j >= m) {
+                    done = true;
+                } else {
+                    i = LIST ? sides[j] : j;
+                    key = keys[i];
+                    q = sample_side(key, pos, nrm, scale, h_svo);
+                    const uint32_t at = start[i];
+                    const D3 mn = v.nmin[at];
+                    d = v.depth[at] + 1u;
+                    sp = 0;
+                    reads = 0;
+                    if (leaf_v(v, at, key)) {
+                        const bool fits = leaf_reliable(mn, sizes[d - 1], q);
+                        if (ci == 0) {
+                            if (LIST) {
+                                skeys[off[i]] = at;
+                                svals[off[i]] = i;
+                            } else {
+                                status[i] = fits ? 1 : 2;
+                                witness[i] = fits ? at : INVALID;
+                                cnt[i] = fits ? 1u : 2u;
+                            }
+                        }
+                    } else {
+                        have = true;
+                        c0 = v.children[at];
+                        px = (float)(mn.x - q.p.x);
+                        py = (float)(mn.y - q.p.y);
+                        pz = (float)(mn.z - q.p.z);
+                        f = SideF(q, fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)) + 2.0f * (float)sizes[d],
+                                  (float)margin);
+                    }
+                }
+            }
+        }
+        if (__all_sync(FULL, done && !have)) break;
+        // ---- the eight children of the node
+        uint32_t ch = INVALID;
+        bool leaf = false, inner = false, fits = false;
+        const float cs = (float)sizes[d];
+        if (have) {
+            const uint32_t idx = c0 + ci;
+            ch = v.children[idx];
+            const bool is_leaf = ch == INVALID || v.cc[idx] >= key;   // leaf_v
+            const float x = (ci & 1u) ? px + cs : px, y = (ci & 2u) ? py + cs : py, z = (ci & 4u) ? pz + cs : pz;
+            const Decision meets = f.box(x, y, z, cs);
+            if (meets == YES || (meets == UNSURE && intersect_side(v.nmin[idx], sizes[d], q))) {
+                leaf = is_leaf;
+                inner = !is_leaf;
+                if (leaf) {
+                    const Decision r = f.reliable(x, y, z, cs);
+                    fits = r == YES || (r == UNSURE && leaf_reliable(v.nmin[idx], sizes[d], q));
+                }
+            }
+        }
+        const unsigned leaves = (__ballot_sync(FULL, leaf) >> shift) & 0xFFu;
+        const unsigned found = (__ballot_sync(FULL, fits) >> shift) & 0xFFu;
+        unsigned left = ((__ballot_sync(FULL, inner) >> shift) & 0xFFu) | found;
+        if (LIST && leaf) {   // a writer rejects them all
+            const uint32_t o = off[i] + reads + __popc(leaves & ((1u << ci) - 1u));
+            skeys[o] = c0 + ci;
+            svals[o] = i;
+        }
+        reads += __popc(leaves);
+        // ---- the lowest child left decides; without one, the stack does
+        bool popped = false;
+        unsigned rel = found;
+        if (have && left == 0 && sp > 0) {
+            const uint64_t e = st[--sp];
+            c0 = (uint32_t)e;
+            left = (unsigned)(e >> 32) & 0xFFu;
+            rel = (unsigned)(e >> 40) & 0xFFu;
+            d = (uint32_t)(e >> 48);
+            popped = true;
+        }
+        const int first = left ? __ffs(left) - 1 : 0;
+        const uint32_t block = __shfl_sync(FULL, ch, (int)shift + first);
+        __syncwarp();   // the stack entry is read
+        if (have) {
+            const uint32_t node = c0 + (uint32_t)first;
+            const bool ends = left == 0 || ((rel >> first) & 1u);
+            if (ends) {
+                have = false;
+                if (!LIST && ci == 0) {
+                    status[i] = left ? 1 : 2;
+                    witness[i] = left ? node : INVALID;
+                    cnt[i] = left ? 1u : reads + 1u;
+                }
+            } else {
+                const unsigned rest = left & (left - 1);
+                if (rest) {
+                    if (sp >= MAX_TREE_DEPTH) {
+                        if (ci == 0) atomicExch(err, 1);
+                        have = false;
+                    } else {
+                        if (ci == 0)
+                            st[sp] = (uint64_t)c0 | ((uint64_t)rest << 32) | ((uint64_t)rel << 40) | ((uint64_t)d << 48);
+                        ++sp;
+                    }
+                }
+                if (popped) {
+                    const D3 mn = v.nmin[node];
+                    c0 = v.children[node];
+                    px = (float)(mn.x - q.p.x);
+                    py = (float)(mn.y - q.p.y);
+                    pz = (float)(mn.z - q.p.z);
+                } else {
+                    c0 = block;
+                    if (first & 1) px += cs;
+                    if (first & 2) py += cs;
+                    if (first & 4) pz += cs;
+                }
+                ++d;
+            }
+        }
+        __syncwarp();   // the stack entry is written
+    }
+}
+
+// The dependency pairs that need no search: a witness, and every writer's descent leaf, its last.
+__global__ void k_sens(uint32_t m, const uint8_t *status, const uint32_t *witness, const uint32_t *dleaf,
+                       const uint32_t *off, uint32_t *skeys, uint32_t *svals) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t o = status[i] == 1 ? off[i] : off[i + 1] - 1;
+    skeys[o] = status[i] == 1 ? witness[i] : dleaf[i];
+    svals[o] = i;
 }
 
 // Conflict resolution of a round as a breadth-first search in key order.
@@ -429,34 +634,6 @@ __global__ void k_waves_coop(uint32_t nf0, uint32_t *front, uint32_t *next, cons
     if (gtid == 0) *waves_out += wave;   // running total over the rounds
 }
 
-// Dependency lists: the leaves each pending side depends on (its witness if
-// reliable; the leaves its search read plus its descent leaf if a writer),
-// written as (leaf, side) pairs at the offsets of the evaluation's counts.
-__global__ void k_sens(uint32_t m, const uint32_t *keys, NV v, Root root, const D3 *pos, const D3 *nrm,
-                       const double *scale, double h_svo, const uint8_t *status, const uint32_t *witness,
-                       const uint32_t *dleaf, const uint32_t *off, uint32_t *skeys, uint32_t *svals, double margin,
-                       int *err) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    if (status[i] == 1) {
-        skeys[off[i]] = witness[i];
-        svals[off[i]] = i;
-        return;
-    }
-    uint32_t key = keys[i];
-    SampleRef q = sample_side(key, pos, nrm, scale, h_svo);
-    int e = 0;
-    uint32_t c = 0, o = off[i];
-    find_reliable_v(v, root, sphere_start_v(v, root, key, q, margin), key, q, [&](uint32_t leaf) {
-        skeys[o + c] = leaf;
-        svals[o + c] = i;
-        ++c;
-    }, &e);
-    skeys[o + c] = dleaf[i];
-    svals[o + c] = i;
-    if (e) atomicExch(err, e);
-}
-
 __global__ void k_writer_list(uint32_t m, const uint8_t *status, uint32_t *writers, uint32_t *nwri) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m && status[i] == 2) writers[atomicAdd(nwri, 1u)] = i;
@@ -495,7 +672,7 @@ __global__ void k_sampling_apply(uint32_t m, const uint32_t *keys, const uint8_t
     }
     uint32_t key = keys[i];
     SampleRef q = sample_side(key, pos, nrm, scale, h_svo);
-    D3 endp = segment_end(q);
+    const Segment seg(q.p, segment_end(q));
     uint32_t node = dleaf[i];
     D3 mn = v.nmin[node];
     uint32_t d = v.depth[node];
@@ -519,7 +696,7 @@ __global__ void k_sampling_apply(uint32_t m, const uint32_t *keys, const uint8_t
             if (phase == 0) nsplit[i] = splits;
             return;
         }
-        uint32_t b = best_child(mn, sz, q.p, endp);
+        uint32_t b = best_child(mn, sz, seg);
         if (b == INVALID) { atomicExch(err, 4); if (phase == 0) nsplit[i] = splits; return; }
         mn = child_coords(mn, cs, b);
         d += 1;
@@ -1176,28 +1353,33 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         } ev;
         for (cudaEvent_t &x : ev.e) TSR_CUDA(cudaEventCreate(&x));
         cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], e2 = ev.e[2];
-        unsigned coop_grid = 1;
+        DBuf<uint32_t> taken(2, st);   // sides the two searches of a round have taken
+        unsigned coop_grid = 1, search_grid = 1;
         {
             int dev = 0, sms = 0, per_sm = 0;
             TSR_CUDA(cudaGetDevice(&dev));
             TSR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_waves_coop, 256, 0));
             coop_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
+            TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<false>, 128, 0));
+            search_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
         }
         const uint32_t max_waves_used = limit_sampling_waves();
         while (m > 0) {
             if (++rounds > limit_rounds()) fail(TSR_ERR_TIMEOUT, "sampling rounds did not converge");
             NV v = view(S);
             DBuf<uint8_t> status(m, st);
-            DBuf<uint32_t> unres(m, st), witness(m, st), dleaf(m, st);
+            DBuf<uint32_t> unres(m, st), witness(m, st), dleaf(m, st), begin(m, st);
             DBuf<uint32_t> scnt(m + 1, st), soff(m + 1, st), writers(m, st);
             unres.zero();
             TSR_CUDA(cudaMemsetAsync(scnt.p + m, 0, 4, st));
             TSR_CUDA(cudaEventRecord(e0, st));
-            k_sampling_eval<<<grid_for(m, 128), 128, 0, st>>>(m, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo,
-                                                             status.p, witness.p, dleaf.p, scnt.p, margin, derr.p,
-                                                             rounds == 1 ? 1 : 0);
-            ::tsr::note_launch();
+            k_sides_begin<<<grid_for(m, 128), 128, 0, st>>>(m, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p,
+                                                           dleaf.p, margin, derr.p); ::tsr::note_launch();
+            taken.zero();
+            k_search<false><<<std::min(search_grid, grid_for(m, 16)), 128, 0, st>>>(
+                m, nullptr, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p, status.p, witness.p, scnt.p, nullptr,
+                nullptr, nullptr, margin, taken.p, derr.p); ::tsr::note_launch();
             TSR_CUDA(cudaEventRecord(e1, st));
             // dependency index (leaf -> sides) and the writer list
             exclusive_scan(scnt.p, soff.p, m + 1, st);
@@ -1210,9 +1392,13 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             const uint32_t nsens = cnt[0], nwri = cnt[1];
             DBuf<uint32_t> skeys(nsens, st), svals(nsens, st), ssorted(nsens, st), by_leaf(nsens, st);
             if (nsens) {
-                k_sens<<<grid_for(m, 128), 128, 0, st>>>(m, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, status.p,
-                                                        witness.p, dleaf.p, soff.p, skeys.p, svals.p, margin,
-                                                        derr.p); ::tsr::note_launch();
+                k_sens<<<grid_for(m, BLK), BLK, 0, st>>>(m, status.p, witness.p, dleaf.p, soff.p, skeys.p, svals.p);
+                ::tsr::note_launch();
+                if (nwri) {
+                    k_search<true><<<std::min(search_grid, grid_for(nwri, 16)), 128, 0, st>>>(
+                        nwri, writers.p, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p, nullptr, nullptr,
+                        nullptr, soff.p, skeys.p, svals.p, margin, taken.p + 1, derr.p); ::tsr::note_launch();
+                }
                 int leaf_bits = 1;   // node indices stay below the node count
                 while (leaf_bits < 32 && (1ull << leaf_bits) < (uint64_t)S.count) ++leaf_bits;
                 sort_pairs(skeys.p, ssorted.p, svals.p, by_leaf.p, nsens, st, leaf_bits);
