@@ -174,79 +174,117 @@ __device__ __forceinline__ void fill_counts(uint32_t n, uint32_t &va, uint32_t &
 
 // FlexibleMesh::findBorderRings / findBorderRing / extendBorderRing /
 // removeDuplicatesInRings (FlexibleMesh.cpp:1617-1732), replayed by one
-// thread.  order[] is the current order of the edge list (position -> edge),
-// pos[] its inverse; the candidates that continue a ring at vertex v are the
-// unused edges starting at v (stails/sids: edges sorted by tail, stable), and
-// the reference takes the one at the smallest current position.  A set that
-// cannot be closed stays one ring, as in the reference.  Ring vertices are
-// the edge tails in ring order; rings of fewer than 3 vertices are counted
-// and not filled (the reference reads past them, FlexibleMesh.cpp:1905-1916).
-__global__ void k_rings(uint32_t nb, const uint32_t *tail, const uint32_t *head, const uint32_t *stails,
-                        const uint32_t *sids, uint32_t *order, uint32_t *pos, uint8_t *used, uint32_t *ring_start,
-                        uint32_t *ring_len, uint32_t *ring_verts, uint32_t *ring_vofs, uint32_t *ring_tofs,
-                        RingOut *out) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (uint32_t j = 0; j < nb; ++j) {
+// thread of one block.  order[] is the current order of the edge list
+// (position -> edge), pos[] its inverse; the candidates that continue a ring
+// at vertex v are the unused edges starting at v (stails/sids: edges sorted by
+// tail, stable), and the reference takes the one at the smallest current
+// position.  A set that cannot be closed stays one ring, as in the reference.
+// Ring vertices are the edge tails in ring order; rings of fewer than 3
+// vertices are counted and not filled (the reference reads past them,
+// FlexibleMesh.cpp:1905-1916).
+//
+// The block finds every edge's first candidate beforehand, and keeps the arrays
+// the thread walks in shared memory where they fit (RINGS_SHARED edges): its
+// chain of dependent loads is what bounds it, 0.9 us an edge from global memory
+// with a binary search in the chain, 0.2 us now.
+constexpr uint32_t RINGS_SHARED = 9000;
+constexpr unsigned RINGS_BLK = 256;
+inline size_t rings_shared_bytes(uint32_t nb) { return nb <= RINGS_SHARED ? (size_t)nb * 25 : 0; }
+
+__global__ void __launch_bounds__(RINGS_BLK)
+k_rings(uint32_t nb, const uint32_t *g_tail, const uint32_t *g_head, const uint32_t *g_stails, const uint32_t *g_sids,
+        uint32_t *g_first, uint32_t *g_order, uint32_t *g_pos, uint8_t *g_used, uint32_t *ring_start,
+        uint32_t *ring_len, uint32_t *ring_verts, uint32_t *ring_vofs, uint32_t *ring_tofs, RingOut *out) {
+    extern __shared__ uint32_t ring_shared[];
+    const uint32_t *head = g_head, *stails = g_stails, *sids = g_sids;
+    uint32_t *first = g_first, *order = g_order, *pos = g_pos;
+    uint8_t *used = g_used;
+    if (nb <= RINGS_SHARED) {
+        uint32_t *s = ring_shared;
+        for (uint32_t j = threadIdx.x; j < nb; j += RINGS_BLK) {
+            s[j] = g_head[j];
+            s[nb + j] = g_stails[j];
+            s[2 * nb + j] = g_sids[j];
+        }
+        head = s;
+        stails = s + nb;
+        sids = s + 2 * nb;
+        first = s + 3 * nb;
+        order = s + 4 * nb;
+        pos = s + 5 * nb;
+        used = reinterpret_cast<uint8_t *>(s + 6 * nb);
+    }
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < nb; j += RINGS_BLK) {
         order[j] = j;
         pos[j] = j;
         used[j] = 0;
-    }
-    uint32_t rings = 0, holes = 0, skipped = 0, add_v = 0, add_t = 0, s0 = 0;
-    while (s0 < nb) {
-        const uint32_t start = tail[order[s0]];
-        used[order[s0]] = 1;
-        uint32_t r = s0 + 1;
-        bool closed = false;
-        while (r < nb) {
-            const uint32_t end = head[order[r - 1]];
-            // edges starting at `end`: lower bound in the tail-sorted index
-            uint32_t lo = 0, hi = nb;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (stails[mid] < end) lo = mid + 1; else hi = mid;
-            }
-            uint32_t best = 0xFFFFFFFFu;
-            for (uint32_t q = lo; q < nb && stails[q] == end; ++q) {
-                const uint32_t id = sids[q];
-                if (!used[id] && pos[id] < best) best = pos[id];
-            }
-            if (best == 0xFFFFFFFFu) break;
-            const uint32_t id = order[best], other = order[r];
-            order[r] = id;
-            pos[id] = r;
-            order[best] = other;
-            pos[other] = best;
-            used[id] = 1;
-            ++r;
-            if (head[id] == start) {
-                closed = true;
-                break;
-            }
+        // edges starting at this one's end: lower bound in the tail-sorted index
+        const uint32_t end = head[j];
+        uint32_t lo = 0, hi = nb;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (stails[mid] < end) lo = mid + 1; else hi = mid;
         }
-        const uint32_t stop = closed ? r : nb;   // an unclosed set stays whole
-        const uint32_t n = stop - s0;
-        ring_start[rings] = s0;
-        ring_len[rings] = n;
-        for (uint32_t p = s0; p < stop; ++p) ring_verts[p] = tail[order[p]];
-        uint32_t va = 0, ta = 0;
-        if (n >= 3) {
-            fill_counts(n, va, ta);
-            ++holes;
-        } else {
-            ++skipped;
-        }
-        ring_vofs[rings] = add_v;
-        ring_tofs[rings] = add_t;
-        add_v += va;
-        add_t += ta;
-        ++rings;
-        s0 = stop;
+        first[j] = lo;
     }
-    out->rings = rings;
-    out->holes = holes;
-    out->skipped = skipped;
-    out->add_v = add_v;
-    out->add_t = add_t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t rings = 0, holes = 0, skipped = 0, add_v = 0, add_t = 0, s0 = 0;
+        while (s0 < nb) {
+            uint32_t last = order[s0];
+            const uint32_t start = g_tail[last];
+            used[last] = 1;
+            uint32_t r = s0 + 1;
+            bool closed = false;
+            while (r < nb) {
+                const uint32_t end = head[last];
+                uint32_t best = 0xFFFFFFFFu;
+                for (uint32_t q = first[last]; q < nb && stails[q] == end; ++q) {
+                    const uint32_t id = sids[q];
+                    if (!used[id] && pos[id] < best) best = pos[id];
+                }
+                if (best == 0xFFFFFFFFu) break;
+                const uint32_t id = order[best], other = order[r];
+                order[r] = id;
+                pos[id] = r;
+                order[best] = other;
+                pos[other] = best;
+                used[id] = 1;
+                last = id;
+                ++r;
+                if (head[id] == start) {
+                    closed = true;
+                    break;
+                }
+            }
+            const uint32_t stop = closed ? r : nb;   // an unclosed set stays whole
+            const uint32_t n = stop - s0;
+            ring_start[rings] = s0;
+            ring_len[rings] = n;
+            uint32_t va = 0, ta = 0;
+            if (n >= 3) {
+                fill_counts(n, va, ta);
+                ++holes;
+            } else {
+                ++skipped;
+            }
+            ring_vofs[rings] = add_v;
+            ring_tofs[rings] = add_t;
+            add_v += va;
+            add_t += ta;
+            ++rings;
+            s0 = stop;
+        }
+        out->rings = rings;
+        out->holes = holes;
+        out->skipped = skipped;
+        out->add_v = add_v;
+        out->add_t = add_t;
+    }
+    __syncthreads();
+    // a ring's part of the order is final once the ring is
+    for (uint32_t j = threadIdx.x; j < nb; j += RINGS_BLK) ring_verts[j] = g_tail[order[j]];
 }
 
 struct RingView {
@@ -491,6 +529,7 @@ void postprocess_mesh(tsr_mesh &m, uint32_t min_isle_size, tsr_mesh_post_counts 
         if (nb) {
             DBuf<uint32_t> tail(nb, st), head(nb, st), stails(nb, st), sids(nb, st), iota(nb, st), order(nb, st),
                 posn(nb, st);
+            DBuf<uint32_t> first(nb, st);
             DBuf<uint8_t> used(nb, st);
             ring_start.alloc(nb, st); ring_len.alloc(nb, st); ring_verts.alloc(nb, st);
             ring_vofs.alloc(nb, st); ring_tofs.alloc(nb, st);
@@ -498,8 +537,12 @@ void postprocess_mesh(tsr_mesh &m, uint32_t min_isle_size, tsr_mesh_post_counts 
             k_border_edges<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, corners.p, tris_p, tail.p, head.p); ::tsr::note_launch();
             k_iota_u32<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, iota.p); ::tsr::note_launch();
             sort_kv(tail.p, stails.p, iota.p, sids.p, nb, bits_for(nvk), st);
-            k_rings<<<1, 1, 0, st>>>(nb, tail.p, head.p, stails.p, sids.p, order.p, posn.p, used.p, ring_start.p,
-                                     ring_len.p, ring_verts.p, ring_vofs.p, ring_tofs.p, out.p); ::tsr::note_launch();
+            const size_t smem = rings_shared_bytes(nb);
+            TSR_CUDA(cudaFuncSetAttribute(k_rings, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)rings_shared_bytes(RINGS_SHARED)));
+            k_rings<<<1, RINGS_BLK, smem, st>>>(nb, tail.p, head.p, stails.p, sids.p, first.p, order.p, posn.p, used.p,
+                                                ring_start.p, ring_len.p, ring_verts.p, ring_vofs.p, ring_tofs.p,
+                                                out.p); ::tsr::note_launch();
             ro = read_scalar(out.p, st);
         }
         pc.holes = ro.holes;
