@@ -132,10 +132,13 @@ static void check_samples(const tsr_samples_view &sv, bool on_device) {
         fail(TSR_ERR_INVALID_ARG, "null sample array");
     if ((uint64_t)sv.count * sv.cams_per_sample >= 0xFFFFFFFFull)
         fail(TSR_ERR_OVERFLOW_U32, "link count must stay below 2^32 - 1 (Samples.h:395-402)");
-    if (!on_device)
-        for (uint32_t i = 0; i < sv.count; ++i)
+    if (!on_device) {
+        uint32_t bad = 0;   // no exit from the loop, so that it vectorizes; the index is looked for on failure
+        for (uint32_t i = 0; i < sv.count; ++i) bad += !(sv.scales[i] > 0.0);
+        for (uint32_t i = 0; bad && i < sv.count; ++i)
             if (!(sv.scales[i] > 0.0))   // Samples.cpp:280-288
                 fail(TSR_ERR_INVALID_ARG, "invalid (non-positive) sample scale at index " + std::to_string(i));
+    }
 }
 
 static tsr_status tree_build_impl(const tsr_samples_view *samples, const tsr_params *params, void *cuda_stream,
@@ -534,7 +537,9 @@ tsr_status tsr_mesh_create(const double *positions, const double *scales, uint64
             fail(TSR_ERR_INVALID_ARG, "null argument");
         if (vertex_count >= INVALID || 3 * triangle_count >= INVALID)
             fail(TSR_ERR_OVERFLOW_U32, "vertex and corner counts must stay below 2^32 - 1");
-        for (uint64_t i = 0; i < 3 * triangle_count; ++i)
+        uint32_t largest = 0;   // as for the scales: one pass that vectorizes
+        for (uint64_t i = 0; i < 3 * triangle_count; ++i) largest = triangles[i] > largest ? triangles[i] : largest;
+        for (uint64_t i = 0; largest >= vertex_count && i < 3 * triangle_count; ++i)
             if (triangles[i] >= vertex_count)
                 fail(TSR_ERR_INVALID_ARG, "triangle index out of range at corner " + std::to_string(i));
         tsr_mesh *m = new tsr_mesh();
