@@ -64,7 +64,7 @@ __global__ void k_classify(uint32_t nc, const uint32_t *cells, const double *occ
     ntri[c] = cnt;
 }
 
-__global__ void k_emit(uint32_t nc, const uint32_t *cells, const double *occ, const uint32_t *toff,
+__global__ void k_emit(uint32_t nc, const uint32_t *cells, const double *occ, const uint32_t *toff, int leaf_bits,
                        uint64_t *keys, uint32_t *vals, uint32_t *ends) {
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
@@ -80,7 +80,7 @@ __global__ void k_emit(uint32_t nc, const uint32_t *cells, const double *occ, co
             uint32_t l0 = leaf[c_ends[e][0]], l1 = leaf[c_ends[e][1]];
             uint32_t g = 3 * slot + j;
             uint32_t lo = l0 < l1 ? l0 : l1, hi = l0 < l1 ? l1 : l0;
-            keys[g] = ((uint64_t)hi << 32) | lo;   // EdgeVertexIndex ordering: max leaf, then min leaf
+            keys[g] = ((uint64_t)hi << leaf_bits) | lo;   // EdgeVertexIndex ordering: max leaf, then min leaf
             vals[g] = g;
             ends[2 * (size_t)g] = l0;
             ends[2 * (size_t)g + 1] = l1;
@@ -156,12 +156,19 @@ void exscan(const T *in, T *out, uint32_t n, cudaStream_t st) {
     TSR_CUDA(cub::DeviceScan::ExclusiveSum(t.p, tmp, in, out, n, st));
 }
 
+// Stable sort on the bits that the keys have.
 template <class K, class V>
-void sortp(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, cudaStream_t st) {
+void sortp(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, int bits, cudaStream_t st) {
     size_t tmp = 0;
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kin, kout, vin, vout, n, 0, sizeof(K) * 8, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kin, kout, vin, vout, n, 0, bits, st));
     DBuf<uint8_t> t(tmp, st);
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kin, kout, vin, vout, n, 0, sizeof(K) * 8, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kin, kout, vin, vout, n, 0, bits, st));
+}
+
+int bits_below(uint32_t n) {
+    int b = 1;
+    while (b < 32 && (1u << b) < n) ++b;
+    return b;
 }
 
 }  // namespace
@@ -189,8 +196,9 @@ void extract_dmc(const tsr_tree &t, const tsr_occupancy &o, tsr_mesh &m) {
     }
     DBuf<uint64_t> keys(mc, st), skeys(mc, st);
     DBuf<uint32_t> vals(mc, st), svals(mc, st), ends(2ull * mc, st);
-    k_emit<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, t.cells.p, o.occ.p, toff.p, keys.p, vals.p, ends.p); ::tsr::note_launch();
-    sortp(keys.p, skeys.p, vals.p, svals.p, mc, st);
+    const int leaf_bits = bits_below(t.n_leaves);
+    k_emit<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, t.cells.p, o.occ.p, toff.p, leaf_bits, keys.p, vals.p, ends.p); ::tsr::note_launch();
+    sortp(keys.p, skeys.p, vals.p, svals.p, mc, 2 * leaf_bits, st);
     DBuf<uint32_t> head(mc, st), segid(mc, st), first(mc, st);
     k_heads<<<grid_for(mc, BLK), BLK, 0, st>>>(mc, skeys.p, svals.p, head.p, first.p); ::tsr::note_launch();
     {
@@ -203,7 +211,7 @@ void extract_dmc(const tsr_tree &t, const tsr_occupancy &o, tsr_mesh &m) {
     m.n_verts = nv;
     DBuf<uint32_t> seg_first(nv, st), seg_iota(nv, st), sfirst(nv, st), order(nv, st), vert_of_seg(nv, st);
     k_seg_first<<<grid_for(mc, BLK), BLK, 0, st>>>(mc, head.p, segid.p, svals.p, seg_first.p, seg_iota.p); ::tsr::note_launch();
-    sortp(seg_first.p, sfirst.p, seg_iota.p, order.p, nv, st);
+    sortp(seg_first.p, sfirst.p, seg_iota.p, order.p, nv, bits_below(mc), st);
     k_rank<<<grid_for(nv, BLK), BLK, 0, st>>>(nv, order.p, vert_of_seg.p); ::tsr::note_launch();
     k_tris<<<grid_for(mc, BLK), BLK, 0, st>>>(mc, svals.p, segid.p, vert_of_seg.p, m.tris.p); ::tsr::note_launch();
     m.vpos.alloc(3ull * nv, st);

@@ -69,12 +69,12 @@ __device__ void uf_unite(uint32_t *parent, uint32_t a, uint32_t b, int *err) {
     atomicExch(err, 2);
 }
 
-__global__ void k_edge_keys(uint32_t nc, const uint32_t *tris, uint64_t *keys, uint32_t *vals) {
+__global__ void k_edge_keys(uint32_t nc, const uint32_t *tris, int vertex_bits, uint64_t *keys, uint32_t *vals) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
     const uint32_t t = c / 3, k = c - 3 * t;
     const uint32_t a = tris[c], b = tris[3 * t + (k == 2 ? 0 : k + 1)];
-    keys[c] = ((uint64_t)min(a, b) << 32) | max(a, b);
+    keys[c] = ((uint64_t)min(a, b) << vertex_bits) | max(a, b);
     vals[c] = c;
 }
 
@@ -85,7 +85,7 @@ __global__ void k_iota_u32(uint32_t n, uint32_t *x) {
 
 // One thread per sorted corner edge; the first of each run of equal keys
 // classifies the edge and joins its vertices' isles.
-__global__ void k_edge_runs(uint32_t nc, const uint64_t *skeys, const uint32_t *svals, uint8_t *border,
+__global__ void k_edge_runs(uint32_t nc, const uint64_t *skeys, int vertex_bits, const uint32_t *svals, uint8_t *border,
                             uint32_t *parent, int *err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
@@ -96,7 +96,7 @@ __global__ void k_edge_runs(uint32_t nc, const uint64_t *skeys, const uint32_t *
     if (i + 2 < nc && skeys[i + 2] == key) ++run;
     if (run >= 3) atomicExch(err, 1);
     if (run == 1) border[svals[i]] = 1;
-    uf_unite(parent, (uint32_t)(key >> 32), (uint32_t)key, err);
+    uf_unite(parent, (uint32_t)(key >> vertex_bits), (uint32_t)(key & ((1ull << vertex_bits) - 1)), err);
 }
 
 __global__ void k_labels(uint32_t nv, uint32_t *parent, uint32_t *label, uint32_t *size, int *err) {
@@ -456,9 +456,10 @@ void postprocess_mesh(tsr_mesh &m, uint32_t min_isle_size, tsr_mesh_post_counts 
     if (nc) {
         DBuf<uint64_t> keys(nc, st), skeys(nc, st);
         DBuf<uint32_t> vals(nc, st), svals(nc, st);
-        k_edge_keys<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, m.tris.p, keys.p, vals.p); ::tsr::note_launch();
-        sort_kv(keys.p, skeys.p, vals.p, svals.p, nc, 64, st);
-        k_edge_runs<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, skeys.p, svals.p, border.p, parent.p, err.p); ::tsr::note_launch();
+        const int vertex_bits = bits_for(nv - 1);   // edges have vertices
+        k_edge_keys<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, m.tris.p, vertex_bits, keys.p, vals.p); ::tsr::note_launch();
+        sort_kv(keys.p, skeys.p, vals.p, svals.p, nc, 2 * vertex_bits, st);
+        k_edge_runs<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, skeys.p, vertex_bits, svals.p, border.p, parent.p, err.p); ::tsr::note_launch();
     }
     if (nv) {
         k_labels<<<grid_for(nv, BLK), BLK, 0, st>>>(nv, parent.p, label.p, size.p, err.p); ::tsr::note_launch();

@@ -717,20 +717,17 @@ __device__ inline uint32_t get_node(const uint32_t *children, const D3 *nmin, co
     D3 mn = root.mn;
     while (true) {
         if (children[node] == INVALID || depth == max_depth) break;
-        double cs = dmul(size, 0.5);
-        uint32_t c0 = children[node];
-        bool moved = false;
-        for (uint32_t c = 0; c < 8; ++c) {
-            D3 cmn = child_coords(mn, cs, c);
-            if (!node_contains(q, cmn, cs, 0.0)) continue;
-            node = c0 + c;
-            mn = cmn;
-            size = cs;
-            ++depth;
-            moved = true;
-            break;
-        }
-        if (!moved) break;
+        // the child whose half-open box holds q: on each axis the boxes of the
+        // two halves share no point, so the half q lies in decides
+        const double cs = dmul(size, 0.5);
+        const D3 mid{dadd(mn.x, cs), dadd(mn.y, cs), dadd(mn.z, cs)};
+        const bool hx = q.x >= mid.x, hy = q.y >= mid.y, hz = q.z >= mid.z;
+        const D3 cmn{hx ? mid.x : mn.x, hy ? mid.y : mn.y, hz ? mid.z : mn.z};
+        if (!node_contains(q, cmn, cs, 0.0)) break;
+        node = children[node] + ((hx ? 1u : 0u) | (hy ? 2u : 0u) | (hz ? 4u : 0u));
+        mn = cmn;
+        size = cs;
+        ++depth;
     }
     *out_depth = depth;
     return node;
@@ -890,23 +887,32 @@ __global__ void k_neighbor_events(uint32_t nl, const uint32_t *leaf_node, const 
     }
 }
 
-__global__ void k_neighbor_pairs(uint32_t ne, const uint32_t *dst, const uint32_t *slot, uint64_t *keys,
-                                 uint32_t *vals) {
-    uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+// Both ends of every edge into their rows, in no order yet: (event, other end).
+__global__ void k_neighbor_entries(uint32_t ne, const uint32_t *dst, const uint32_t *off, uint32_t *used,
+                                   uint2 *entries) {
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
-    uint32_t o = dst[e];
+    const uint32_t o = dst[e];
     if (o == INVALID) return;
-    uint32_t l = e / 6;
-    uint32_t j = 2 * slot[e];
-    keys[j] = ((uint64_t)l << 32) | e;
-    vals[j] = o;
-    keys[j + 1] = ((uint64_t)o << 32) | e;
-    vals[j + 1] = l;
+    const uint32_t l = e / 6;
+    entries[off[l] + atomicAdd(&used[l], 1u)] = make_uint2(e, o);
+    entries[off[o] + atomicAdd(&used[o], 1u)] = make_uint2(e, l);
 }
 
-__global__ void k_valid_flags(uint32_t n, const uint32_t *dst, uint32_t *flag) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) flag[i] = dst[i] != INVALID ? 1u : 0u;
+// A row's entries in the order of their events: a row has about seven, so an
+// entry's rank by counting the smaller ones beats sorting all (leaf, event)
+// pairs by their 64 bits in 8 passes (the stage, with the octant descent of
+// get_node: 7.1 -> 1.8 ms at 16M samples, 0.24 -> 0.08 ms at 4k).
+__global__ void k_neighbor_rows(uint32_t nl, const uint32_t *off, const uint2 *entries, uint32_t *nbs) {
+    const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= nl) return;
+    const uint32_t lo = off[l], hi = off[l + 1];
+    for (uint32_t i = lo; i < hi; ++i) {
+        const uint2 x = entries[i];
+        uint32_t rank = lo;
+        for (uint32_t j = lo; j < hi; ++j) rank += entries[j].x < x.x;
+        nbs[rank] = x.y;
+    }
 }
 
 // -------------------------------------------------------------- dual cells
@@ -1064,24 +1070,26 @@ __device__ void expand_frame(uint8_t type, const uint32_t *nd, uint64_t khi, uin
 }
 
 __global__ void k_frames_count(uint32_t m, const uint8_t *type, const uint32_t *nodes, uint32_t level,
-                               const uint32_t *children, const uint32_t *node_to_leaf, uint32_t *nf, uint32_t *nc) {
+                               const uint32_t *children, const uint32_t *node_to_leaf, uint64_t *counts) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
+    if (i > m) return;
+    if (i == m) {   // the scan's last entry becomes the totals
+        counts[m] = 0;
+        return;
+    }
     uint32_t fo = 0, co = 0;
     expand_frame<false>(type[i], nodes + 8 * (size_t)i, 0, 0, level, children, node_to_leaf, fo, co, nullptr, nullptr,
                         nullptr, nullptr, nullptr, nullptr, nullptr);
-    nf[i] = fo;
-    nc[i] = co;
+    counts[i] = ((uint64_t)co << 32) | fo;   // cells, frames: one scan for both
 }
 
 __global__ void k_frames_write(uint32_t m, const uint8_t *type, const uint32_t *nodes, const uint64_t *khi,
                                const uint64_t *klo, uint32_t level, const uint32_t *children,
-                               const uint32_t *node_to_leaf, const uint32_t *foff, const uint32_t *coff,
-                               uint32_t cbase, uint8_t *otype, uint32_t *onodes, uint64_t *okhi, uint64_t *oklo,
+                               const uint32_t *node_to_leaf, const uint64_t *offsets, uint32_t cbase, uint8_t *otype, uint32_t *onodes, uint64_t *okhi, uint64_t *oklo,
                                uint32_t *cells, uint64_t *ckhi, uint64_t *cklo) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    uint32_t fo = foff[i], co = cbase + coff[i];
+    uint32_t fo = (uint32_t)offsets[i], co = cbase + (uint32_t)(offsets[i] >> 32);
     expand_frame<true>(type[i], nodes + 8 * (size_t)i, khi[i], klo[i], level, children, node_to_leaf, fo, co, otype,
                        onodes, okhi, oklo, cells, ckhi, cklo);
 }
@@ -1109,6 +1117,14 @@ __global__ void k_iota(uint32_t n, uint32_t *a) {
 }
 
 // ------------------------------------------------------------- cub helpers
+// Key bits of values below n.
+inline int bits_below(uint64_t n) {
+    int b = 1;
+    while (b < 32 && (1ull << b) < n) ++b;
+    return b;
+}
+static_assert(MAX_TREE_DEPTH < 64, "depth keys are 6 bits");
+
 template <class T>
 void exclusive_scan(const T *in, T *out, uint32_t n, cudaStream_t st) {
     size_t tmp = 0;
@@ -1118,11 +1134,12 @@ void exclusive_scan(const T *in, T *out, uint32_t n, cudaStream_t st) {
 }
 
 template <class K, class V>
-void sort_pairs(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, cudaStream_t st, int end_bit = sizeof(K) * 8) {
+void sort_pairs(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, cudaStream_t st, int end_bit = sizeof(K) * 8,
+                int begin_bit = 0) {
     size_t tmp = 0;
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kin, kout, vin, vout, n, 0, end_bit, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kin, kout, vin, vout, n, begin_bit, end_bit, st));
     DBuf<uint8_t> t(tmp, st);
-    TSR_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kin, kout, vin, vout, n, 0, end_bit, st));
+    TSR_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, kin, kout, vin, vout, n, begin_bit, end_bit, st));
 }
 
 template <class T, class F>
@@ -1399,9 +1416,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
                         nwri, writers.p, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p, nullptr, nullptr,
                         nullptr, soff.p, skeys.p, svals.p, margin, taken.p + 1, derr.p); ::tsr::note_launch();
                 }
-                int leaf_bits = 1;   // node indices stay below the node count
-                while (leaf_bits < 32 && (1ull << leaf_bits) < (uint64_t)S.count) ++leaf_bits;
-                sort_pairs(skeys.p, ssorted.p, svals.p, by_leaf.p, nsens, st, leaf_bits);
+                sort_pairs(skeys.p, ssorted.p, svals.p, by_leaf.p, nsens, st, bits_below(S.count));
                 k_segments<<<grid_for(nsens, BLK), BLK, 0, st>>>(nsens, ssorted.p, seg_lo.p, seg_hi.p); ::tsr::note_launch();
             }
             // waves: the frontier starts with every writer
@@ -1532,7 +1547,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         DBuf<uint32_t> iota(nn, st), order(nn, st);
         DBuf<uint8_t> sdepth(nn, st);
         k_iota<<<grid_for(nn, BLK), BLK, 0, st>>>(nn, iota.p); ::tsr::note_launch();
-        sort_pairs(S.depth.p, sdepth.p, iota.p, order.p, nn, st, 8);
+        sort_pairs(S.depth.p, sdepth.p, iota.p, order.p, nn, st, 6);   // depths stay below MAX_TREE_DEPTH
         uint8_t dmax = read_scalar(sdepth.p + nn - 1, st);
         max_depth = dmax;
         DBuf<uint32_t> lstart(dmax + 2, st);
@@ -1570,7 +1585,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
     {
         DBuf<uint32_t> keys(n, st), vals(n, st), skeys(n, st), old_of_new(n, st);
         k_sample_keys<<<grid_for(n, BLK), BLK, 0, st>>>(n, container.p, new_idx.p, keys.p, vals.p); ::tsr::note_launch();
-        sort_pairs(keys.p, skeys.p, vals.p, old_of_new.p, n, st);
+        sort_pairs(keys.p, skeys.p, vals.p, old_of_new.p, n, st, bits_below(nn));
         t.target.alloc(n, st); t.pos.alloc(n, st); t.nrm.alloc(n, st); t.scale.alloc(n, st); t.conf.alloc(n, st);
         t.links.alloc((size_t)n * k, st);
         k_permute_samples<<<grid_for(n, BLK), BLK, 0, st>>>(n, k, old_of_new.p, t.target.p, pos.p, nrm.p, scale.p, conf.p,
@@ -1584,23 +1599,22 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         uint64_t ne64 = (uint64_t)nl * 6;
         if (ne64 >= INVALID) fail(TSR_ERR_OVERFLOW_U32, "too many leaves for the neighbour graph");
         uint32_t ne = (uint32_t)ne64;
-        DBuf<uint32_t> dst(ne, st), rowc(nl + 1, st), flag(ne + 1, st), slot(ne + 1, st);
+        DBuf<uint32_t> dst(ne, st), rowc(nl + 1, st);
         rowc.zero();
         k_neighbor_events<<<grid_for(ne, 128), 128, 0, st>>>(nl, t.leaf_node.p, t.leaf_min.p, t.children.p, t.nmin.p,
                                                             t.depth.p, t.node_to_leaf.p, root, dst.p, rowc.p); ::tsr::note_launch();
         t.nb_off.alloc(nl + 1, st);
         exclusive_scan(rowc.p, t.nb_off.p, nl + 1, st);
-        k_valid_flags<<<grid_for(ne, BLK), BLK, 0, st>>>(ne, dst.p, flag.p); ::tsr::note_launch();
-        TSR_CUDA(cudaMemsetAsync(flag.p + ne, 0, 4, st));
-        exclusive_scan(flag.p, slot.p, ne + 1, st);
-        uint32_t nev = read_scalar(slot.p + ne, st);
-        uint64_t nent = 2ull * nev;
+        // two entries an edge: 12 per leaf at most, and the offsets are 32-bit, as the events are
+        const uint32_t nent = read_scalar(t.nb_off.p + nl, st);
         t.n_nb = nent;
-        DBuf<uint64_t> keys(nent, st), skeys(nent, st);
-        DBuf<uint32_t> vals(nent, st);
+        DBuf<uint2> entries(nent, st);
         t.nbs.alloc(nent, st);
-        k_neighbor_pairs<<<grid_for(ne, BLK), BLK, 0, st>>>(ne, dst.p, slot.p, keys.p, vals.p); ::tsr::note_launch();
-        if (nent) sort_pairs(keys.p, skeys.p, vals.p, t.nbs.p, (uint32_t)nent, st);
+        rowc.zero();
+        if (nent) {
+            k_neighbor_entries<<<grid_for(ne, BLK), BLK, 0, st>>>(ne, dst.p, t.nb_off.p, rowc.p, entries.p); ::tsr::note_launch();
+            k_neighbor_rows<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, t.nb_off.p, entries.p, t.nbs.p); ::tsr::note_launch();
+        }
     }
     t.stage_ms[4] = timer.lap();
 
@@ -1609,7 +1623,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         if (max_depth + 1 > 24) fail(TSR_ERR_OVERFLOW_U32, "tree too deep for the dual-cell path keys");
         DBuf<uint32_t> all_cells;
         DBuf<uint64_t> all_hi, all_lo;
-        uint32_t ncells = 0, ccap = 0;
+        uint32_t ncells = 0, ccap = 0, levels = 0;
         FrameBuf cur_f;
         uint32_t nf = 0;
         if (t.n_nodes > 1) {
@@ -1626,17 +1640,13 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         }
         for (uint32_t level = 0; nf > 0; ++level) {
             if (level >= 24) fail(TSR_ERR_OVERFLOW_U32, "dual-cell recursion deeper than supported");
-            DBuf<uint32_t> cf(nf + 1, st), cc(nf + 1, st), of(nf + 1, st), oc(nf + 1, st);
-            TSR_CUDA(cudaMemsetAsync(cf.p + nf, 0, 4, st));
-            TSR_CUDA(cudaMemsetAsync(cc.p + nf, 0, 4, st));
-            k_frames_count<<<grid_for(nf, 128), 128, 0, st>>>(nf, cur_f.type.p, cur_f.nodes.p, level, t.children.p,
-                                                             t.node_to_leaf.p, cf.p, cc.p); ::tsr::note_launch();
-            exclusive_scan(cf.p, of.p, nf + 1, st);
-            exclusive_scan(cc.p, oc.p, nf + 1, st);
-            uint32_t tot[2];
-            TSR_CUDA(cudaMemcpyAsync(&tot[0], of.p + nf, 4, cudaMemcpyDeviceToHost, st));
-            TSR_CUDA(cudaMemcpyAsync(&tot[1], oc.p + nf, 4, cudaMemcpyDeviceToHost, st));
-            TSR_CUDA(cudaStreamSynchronize(st));
+            DBuf<uint64_t> counts(nf + 1, st), offsets(nf + 1, st);
+            k_frames_count<<<grid_for(nf + 1, 128), 128, 0, st>>>(nf, cur_f.type.p, cur_f.nodes.p, level, t.children.p,
+                                                                 t.node_to_leaf.p, counts.p); ::tsr::note_launch();
+            exclusive_scan(counts.p, offsets.p, nf + 1, st);
+            const uint64_t both = read_scalar(offsets.p + nf, st);
+            const uint32_t tot[2] = {(uint32_t)both, (uint32_t)(both >> 32)};
+            ++levels;
             if ((uint64_t)ncells + tot[1] > ccap) {
                 uint64_t ncap = std::max<uint64_t>((uint64_t)ncells + tot[1], (uint64_t)ccap * 2);
                 if (ncap * 8 >= INVALID) fail(TSR_ERR_OVERFLOW_U32, "too many dual cells");
@@ -1653,7 +1663,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             FrameBuf nx;
             nx.type.alloc(tot[0], st); nx.nodes.alloc((size_t)tot[0] * 8, st); nx.khi.alloc(tot[0], st); nx.klo.alloc(tot[0], st);
             k_frames_write<<<grid_for(nf, 128), 128, 0, st>>>(nf, cur_f.type.p, cur_f.nodes.p, cur_f.khi.p, cur_f.klo.p,
-                                                             level, t.children.p, t.node_to_leaf.p, of.p, oc.p, ncells,
+                                                             level, t.children.p, t.node_to_leaf.p, offsets.p, ncells,
                                                              nx.type.p, nx.nodes.p, nx.khi.p, nx.klo.p, all_cells.p,
                                                              all_hi.p, all_lo.p); ::tsr::note_launch();
             ncells += tot[1];
@@ -1666,11 +1676,17 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             DBuf<uint32_t> idx(ncells, st), idx2(ncells, st), idx3(ncells, st);
             DBuf<uint64_t> k2(ncells, st), k3(ncells, st);
             k_iota<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx.p); ::tsr::note_launch();
-            // LSD: stable sort by the low word, then by the high word
-            sort_pairs(all_lo.p, k2.p, idx.p, idx2.p, ncells, st);
-            DBuf<uint64_t> hi_sorted(ncells, st);
-            k_gather_u64<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx2.p, all_hi.p, hi_sorted.p); ::tsr::note_launch();
-            sort_pairs(hi_sorted.p, k3.p, idx2.p, idx3.p, ncells, st);
+            // A path has 5 bits a level from the top of the high word down.  Up to
+            // 12 levels it lies in the high word alone, in its top 5 * levels bits;
+            // below that the low word is sorted first (stable).
+            const bool deep = levels > 12;
+            if (deep) {
+                sort_pairs(all_lo.p, k2.p, idx.p, idx2.p, ncells, st, 64, 64 - 5 * ((int)levels - 12));
+                k_gather_u64<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx2.p, all_hi.p, k3.p); ::tsr::note_launch();
+                sort_pairs(k3.p, k2.p, idx2.p, idx3.p, ncells, st, 64, 4);
+            } else {
+                sort_pairs(all_hi.p, k2.p, idx.p, idx3.p, ncells, st, 64, 64 - 5 * (int)levels);
+            }
             k_gather_cells<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx3.p, all_cells.p, t.cells.p); ::tsr::note_launch();
         }
     }
