@@ -832,7 +832,7 @@ struct PriorIn {
 
 constexpr int PP_STACK = 28 * MAX_TREE_DEPTH + 32;   // a step pops four blocks and pushes at most 32
 constexpr int PP_LEAVES = 64;   // blocks whose leaves wait; worked off when fewer than 32 are free
-constexpr int PP_TIES = 64;     // leaves that touch a sphere; likewise
+constexpr int PP_TIES = 96;     // leaves that touch a sphere; worked off when fewer than 64 are free
 constexpr int PP_WARPS = 4;
 
 // Occupancy::computePriors (Occupancy.cpp:530-568) with a
@@ -861,13 +861,14 @@ constexpr int PP_WARPS = 4;
 // (in practice a box that touches a sphere) is decided by the FP64 boxes, as
 // the reference does.
 //
-// Measured, all queries of the field: 493 -> 183 ms at 16M held-out samples
-// (7.6M leaves), 34 -> 14.5 ms at 4M CSG samples, 1.5 -> 0.5 ms at 4k sphere
-// samples.  A query per lane read eight records and eight psum rows of its own
-// per expansion, 128 + 256 cache lines a warp's step, and the L1 passed 0.7
-// child tests a clock and SM; here the lines are shared, a test costs 12 of a
-// lane's instructions, and what bounds it is the issue of four warps per
-// scheduler (126 registers; five warps spill and are no faster).  The eight
+// Measured, all queries of the field: 493 -> 168 ms at 16M held-out samples
+// (7.6M leaves), 62 -> 28.6 ms at 300k, 34 -> 13.4 ms at 4M CSG samples, 1.5 ->
+// 0.5 ms at 4k sphere samples.  A query per lane read eight records and eight
+// psum rows of its own per expansion, 128 + 256 cache lines a warp's step, and
+// the L1 passed 0.7 child tests a clock and SM; here the lines are shared and a
+// test costs 12 of a lane's instructions.  What bounds it is latency at four
+// warps a scheduler (126 registers, 32 of them the sums): two leaves a lane at a
+// time are 8 % faster than one, three warps 23 % slower, five spill.  The eight
 // spheres test 1.6 times the boxes one does.
 //
 // BOUNDS (the pruned field's sign certificates): a node that straddles a
@@ -1059,7 +1060,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
         // whole-numbered distances: undecided only when zero
         const bool whole = in.whole_radius && !in.deep && 4.0f * ru * P.ea < 0.125f;
         while (sp > 0 || waiting > 0 || ties > 0) {
-            if (ties > PP_TIES - 32 || (sp == 0 && waiting == 0)) {
+            if (ties > PP_TIES - 64 || (sp == 0 && waiting == 0)) {
                 // ---- leaves that touch a sphere: a lane each
                 for (int j = lane; j < ties; j += 32) {
                     const uint32_t node = w.tie_node[j];
@@ -1081,59 +1082,80 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
                 continue;
             }
             if (waiting > PP_LEAVES - 32 || sp == 0) {
-                // ---- the leaves of the waiting blocks
+                // ---- the leaves of the waiting blocks, two a lane at a time
                 do {
-                    const bool valid = quarter < waiting;
-                    const int at = valid ? waiting - 1 - quarter : 0;
-                    const uint32_t node = 1 + 8 * w.leaf_block[at] + ci;
-                    const float4 B = w.leaf_box[at];
-                    double2 v = make_double2(0.0, 0.0);
-                    if (valid) v = __ldg(&in.psum[node]);
-                    const Box box = box_of(in, P, node, B.x, B.y, B.z, B.w, bx, by, bz);
-                    float s[8];
-                    near_distances(box, r4, s);
-                    bool unsure;
-                    if (whole) {
-                        float product = s[0];
+                    uint32_t node[2];
+                    float4 B[2];
+                    double2 v[2];
 #pragma unroll
-                        for (int q = 1; q < 8; ++q) product *= s[q];
-                        unsure = !(fabsf(product) > 0.0f);
-                    } else {
-                        float least = fabsf(s[0]);
-#pragma unroll
-                        for (int q = 1; q < 8; ++q) least = fminf(least, fabsf(s[q]));
-                        unsure = !(least > 4.0f * distance_error(box.e, ru));
+                    for (int k = 0; k < 2; ++k) {
+                        const int left = waiting - 4 * k;
+                        const bool valid = quarter < left;
+                        const int at = valid ? left - 1 - quarter : 0;
+                        node[k] = 1 + 8 * w.leaf_block[at] + ci;
+                        B[k] = w.leaf_box[at];
+                        v[k] = make_double2(0.0, 0.0);
+                        if (valid) v[k] = __ldg(&in.psum[node[k]]);
                     }
-                    unsure = unsure && (v.x != 0.0 || v.y != 0.0);
-                    const unsigned um = __ballot_sync(FULL, unsure);
-                    if (unsure) {   // decided later, not met here
-                        const float tol = 4.0f * distance_error(box.e, ru);
-                        unsigned ask = 0;
+                    float s[2][8], e[2];
+                    bool unsure[2];
 #pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            if (!(fabsf(s[q]) > tol)) {
-                                ask |= 1u << q;
-                                s[q] = 1.0f;
+                    for (int k = 0; k < 2; ++k) {
+                        const Box box = box_of(in, P, node[k], B[k].x, B[k].y, B[k].z, B[k].w, bx, by, bz);
+                        e[k] = box.e;
+                        near_distances(box, r4, s[k]);
+                        if (whole) {
+                            float product = s[k][0];
+#pragma unroll
+                            for (int q = 1; q < 8; ++q) product *= s[k][q];
+                            unsure[k] = !(fabsf(product) > 0.0f);
+                        } else {
+                            float least = fabsf(s[k][0]);
+#pragma unroll
+                            for (int q = 1; q < 8; ++q) least = fminf(least, fabsf(s[k][q]));
+                            unsure[k] = !(least > 4.0f * distance_error(box.e, ru));
+                        }
+                        unsure[k] = unsure[k] && (v[k].x != 0.0 || v[k].y != 0.0);
+                    }
+                    if (__any_sync(FULL, unsure[0] || unsure[1])) {
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const unsigned um = __ballot_sync(FULL, unsure[k]);
+                            if (unsure[k]) {   // decided later, not met here
+                                const float tol = 4.0f * distance_error(e[k], ru);
+                                unsigned ask = 0;
+#pragma unroll
+                                for (int q = 0; q < 8; ++q)
+                                    if (!(fabsf(s[k][q]) > tol)) {
+                                        ask |= 1u << q;
+                                        s[k][q] = 1.0f;
+                                    }
+                                const int j = ties + __popc(um & below);
+                                w.tie_node[j] = node[k];
+                                w.tie_mask[j] = (uint8_t)(ask & mask);
                             }
-                        const int j = ties + __popc(um & below);
-                        w.tie_node[j] = node;
-                        w.tie_mask[j] = (uint8_t)(ask & mask);
+                            ties += __popc(um);
+                        }
                     }
-                    ties += __popc(um);
                     if (finite) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) add_where_negative(s[q], v, aE[q], aS[q]);
+                        for (int q = 0; q < 8; ++q) {
+                            add_where_negative(s[0][q], v[0], aE[q], aS[q]);
+                            add_where_negative(s[1][q], v[1], aE[q], aS[q]);
+                        }
                     } else {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            if (s[q] < 0.0f) {
-                                aE[q] += v.x / PP_UNIT;
-                                aS[q] += v.y / PP_UNIT;
-                            }
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                if (s[k][q] < 0.0f) {
+                                    aE[q] += v[k].x / PP_UNIT;
+                                    aS[q] += v[k].y / PP_UNIT;
+                                }
                     }
-                    tested += 32;
-                    waiting -= 4;
-                } while ((waiting >= 4 || (waiting > 0 && sp == 0)) && ties <= PP_TIES - 32);
+                    tested += 64;
+                    waiting -= 8;
+                } while ((waiting >= 8 || (waiting > 0 && sp == 0)) && ties <= PP_TIES - 64);
                 if (waiting < 0) waiting = 0;
                 __syncwarp();
                 continue;
