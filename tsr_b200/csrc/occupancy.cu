@@ -883,6 +883,9 @@ struct Packet {   // the block of queries a warp works on
     double size;
     float ea;                  // bound of a corner's distance from its lattice point
     uint32_t q0, max_depth;
+    // the box of the queries' centres: middle and half extent, 4 where both
+    // halves of an axis hold one, 0 at +-4 where one does
+    float mid[3], ext[3];
 };
 
 struct Box {
@@ -1040,6 +1043,13 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
             k.cy = -(Q.y + half) * k.scale;
             k.cz = -(Q.z + half) * k.scale;
             k.ea = (float)(in.corner_error / k.size) * 8.0f;
+            const unsigned low[3] = {mask & 0x55u, mask & 0x33u, mask & 0x0Fu},
+                           high[3] = {mask & 0xAAu, mask & 0xCCu, mask & 0xF0u};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                k.ext[a] = low[a] && high[a] ? 4.0f : 0.0f;
+                k.mid[a] = low[a] && high[a] ? 0.0f : (high[a] ? 4.0f : -4.0f);
+            }
             w.packet = k;
             w.stack[0] = w.leaf_block[0] = 0;
             w.leaf_box[0] = make_float4(k.cx, k.cy, k.cz, __uint_as_float((126u + k.max_depth) << 23));
@@ -1174,10 +1184,11 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
                 const uint32_t d = __float_as_uint(B.w), k = P.max_depth - d;
                 const Box box = box_of(in, P, node, fmaf(B.x, P.scale, P.cx), fmaf(B.y, P.scale, P.cy),
                                        fmaf(B.z, P.scale, P.cz), __uint_as_float((127u + k) << 23), bx, by, bz);
-                const float m = 4.0f + box.h + box.e;
-                const float fx = fabsf(box.x) + m, fy = fabsf(box.y) + m, fz = fabsf(box.z) + m;
-                const float nx = fmaxf(fabsf(box.x) - m, 0.0f), ny = fmaxf(fabsf(box.y) - m, 0.0f),
-                            nz = fmaxf(fabsf(box.z) - m, 0.0f);
+                const float m = box.h + box.e;
+                const float dx = fabsf(box.x - P.mid[0]), dy = fabsf(box.y - P.mid[1]), dz = fabsf(box.z - P.mid[2]);
+                const float mx = P.ext[0] + m, my = P.ext[1] + m, mz = P.ext[2] + m;
+                const float fx = dx + mx, fy = dy + my, fz = dz + mz;
+                const float nx = fmaxf(dx - mx, 0.0f), ny = fmaxf(dy - my, 0.0f), nz = fmaxf(dz - mz, 0.0f);
                 const bool apart = nx * nx + ny * ny + nz * nz > r2 * (1.0f + 1e-6f);
                 const bool inside = fx * fx + fy * fy + fz * fz < r2 * (1.0f - 2e-6f);
                 if (inside && k < (uint32_t)PK) {
