@@ -861,7 +861,7 @@ constexpr int PP_WARPS = 4;
 // (in practice a box that touches a sphere) is decided by the FP64 boxes, as
 // the reference does.
 //
-// Measured, all queries of the field: 493 -> 168 ms at 16M held-out samples
+// Measured, all queries of the field: 493 -> 164 ms at 16M held-out samples
 // (7.6M leaves), 62 -> 28.6 ms at 300k, 34 -> 13.4 ms at 4M CSG samples, 1.5 ->
 // 0.5 ms at 4k sphere samples.  A query per lane read eight records and eight
 // psum rows of its own per expansion, 128 + 256 cache lines a warp's step, and

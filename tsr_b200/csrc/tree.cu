@@ -590,6 +590,8 @@ __global__ void k_sens(uint32_t m, const uint8_t *status, const uint32_t *witnes
     svals[o] = i;
 }
 
+constexpr uint32_t WAVE_THREADS = 1024;
+
 // Conflict resolution of a round as a breadth-first search in key order.
 // A side is unresolved when a leaf it depends on (its witness if reliable;
 // every leaf its search read and its descent leaf if it is a writer) is
@@ -597,53 +599,54 @@ __global__ void k_sens(uint32_t m, const uint8_t *status, const uint32_t *witnes
 // wave from the writers.  The result is the least fixed point, i.e. exactly
 // what a sequential pass in key order computes.
 
-// Each wave: members claim their descent leaf with their key (leaves whose
-// claim dropped are recorded), then every side depending on a recorded leaf
-// with a larger key becomes unresolved and joins the next wave.
+// A wave is a frontier of (descent leaf, key) pairs.  Each lowers its leaf's
+// claim to its key; if that dropped it, the sides that depend on the leaf and
+// have a larger key become unresolved and are the next frontier.  A leaf whose
+// claim drops twice in a wave is followed twice, and the later, smaller key
+// finds all that the larger one would: the frontier is the same set whatever
+// the order, and a wave needs one grid-wide barrier.  All waves of one round
+// run in one cooperative launch; their number is bounded.  The three counters
+// take turns: a wave adds to one, the next wave's is cleared meanwhile, and
+// the third was read before the last barrier.
 //
-// All waves of one round in one cooperative launch (grid-wide barriers
-// instead of a host round trip per wave).  Counter pairs alternate by wave
-// parity; the idle pair is cleared between the two barriers of a wave, when
-// no thread can still be reading it.  The wave count is bounded.
-__global__ void k_waves_coop(uint32_t nf0, uint32_t *front, uint32_t *next, const uint32_t *keys,
-                             const uint32_t *dleaf, uint32_t *mark, uint32_t *touched, const uint32_t *seg_lo,
-                             const uint32_t *seg_hi, const uint32_t *by_leaf, uint32_t *unres, uint32_t *ctr,
-                             uint32_t max_waves, uint32_t *waves_out, int *err) {
+// Most waves are a few hundred pairs, and what bounds them is a chain of eight
+// dependent loads and atomics and the barrier, whose cost grows with the
+// blocks: one block of 1024 threads a SM instead of eight of 256, and a warp a
+// pair (a leaf's list is long: 8 lanes 9.4, 16 lanes 7.9, 32 lanes 7.2 ms of
+// resolution at 4M CSG samples).  Measured, a wave 20 -> 10 us there (471
+// waves in 20 rounds, resolution 12.1 -> 7.2 ms), 9.9 -> 7.4 ms at 16M held-out
+// samples.  Two blocks a SM, or two sides a lane at a time, give nothing.
+__global__ void __launch_bounds__(WAVE_THREADS)
+    k_waves_coop(uint32_t nf0, uint2 *front, uint2 *next, const uint32_t *keys, const uint32_t *dleaf, uint32_t *mark,
+                 const uint32_t *seg_lo, const uint32_t *seg_hi, const uint32_t *by_leaf, uint32_t *unres,
+                 uint32_t *ctr, uint32_t max_waves, uint32_t *waves_out, int *err) {
     cg::grid_group grid = cg::this_grid();
-    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t gsize = gridDim.x * blockDim.x;
-    const uint32_t lane = threadIdx.x & 31, gwarp = gtid >> 5, nwarps = gsize >> 5;
-    uint32_t nf = nf0;
-    uint32_t wave = 0;
+    const uint32_t gtid = blockIdx.x * WAVE_THREADS + threadIdx.x, warps = gridDim.x * (WAVE_THREADS / 32);
+    const unsigned lane = threadIdx.x & 31;
+    uint32_t nf = nf0, wave = 0, at = 0;
     while (nf > 0) {
         if (wave >= max_waves) {
             if (gtid == 0) atomicExch(err, 7);
             break;
         }
-        uint32_t *c = ctr + 2 * (wave & 1);        // this wave's (touched, next) counters
-        uint32_t *c_idle = ctr + 2 * ((wave + 1) & 1);
-        for (uint32_t i = gtid; i < nf; i += gsize) {
-            uint32_t p = front[i];
-            uint32_t x = dleaf[p], k = keys[p];
-            uint32_t old = atomicMin(&mark[x], k);
-            if (old > k) touched[atomicAdd(&c[0], 1u)] = x;
-        }
-        grid.sync();
-        if (gtid == 0) { c_idle[0] = 0; c_idle[1] = 0; }
-        const uint32_t nt = c[0];
-        for (uint32_t j = gwarp; j < nt; j += nwarps) {
-            uint32_t x = touched[j];
-            uint32_t lo = seg_lo[x];
-            if (lo == INVALID) continue;
-            uint32_t hi = seg_hi[x], mk = mark[x];
-            for (uint32_t q2 = lo + lane; q2 < hi; q2 += 32) {
-                uint32_t q = by_leaf[q2];
-                if (keys[q] > mk && atomicExch(&unres[q], 1u) == 0u) next[atomicAdd(&c[1], 1u)] = q;
+        uint32_t *count = ctr + at;
+        at = at == 2 ? 0 : at + 1;
+        if (gtid == 0) ctr[at] = 0;
+        for (uint32_t i = gtid / 32; i < nf; i += warps) {
+            const uint2 pair = front[i];
+            const uint32_t lo = seg_lo[pair.x], hi = seg_hi[pair.x];
+            uint32_t old = 0;
+            if (lane == 0) old = atomicMin(&mark[pair.x], pair.y);
+            old = __shfl_sync(0xffffffffu, old, 0);
+            if (old <= pair.y || lo == INVALID) continue;
+            for (uint32_t j = lo + lane; j < hi; j += 32) {
+                const uint32_t q = by_leaf[j], key = keys[q], x = dleaf[q];
+                if (key > pair.y && atomicExch(&unres[q], 1u) == 0u) next[atomicAdd(count, 1u)] = make_uint2(x, key);
             }
         }
         grid.sync();
-        nf = c[1];
-        uint32_t *tmp = front;
+        nf = *count;
+        uint2 *tmp = front;
         front = next;
         next = tmp;
         ++wave;
@@ -651,9 +654,14 @@ __global__ void k_waves_coop(uint32_t nf0, uint32_t *front, uint32_t *next, cons
     if (gtid == 0) *waves_out += wave;   // running total over the rounds
 }
 
-__global__ void k_writer_list(uint32_t m, const uint8_t *status, uint32_t *writers, uint32_t *nwri) {
+// The writers, and as pairs of descent leaf and key the first frontier.
+__global__ void k_writer_list(uint32_t m, const uint8_t *status, const uint32_t *keys, const uint32_t *dleaf,
+                              uint32_t *writers, uint2 *front, uint32_t *nwri) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m && status[i] == 2) writers[atomicAdd(nwri, 1u)] = i;
+    if (i >= m || status[i] != 2) return;
+    const uint32_t at = atomicAdd(nwri, 1u);
+    writers[at] = i;
+    front[at] = make_uint2(dleaf[i], keys[i]);
 }
 
 __global__ void k_segments(uint32_t n, const uint32_t *sorted, uint32_t *seg_lo, uint32_t *seg_hi) {
@@ -1393,8 +1401,7 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             int dev = 0, sms = 0, per_sm = 0;
             TSR_CUDA(cudaGetDevice(&dev));
             TSR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_waves_coop, 256, 0));
-            coop_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
+            coop_grid = (unsigned)sms;   // a block a SM
             TSR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search<false>, 128, 0));
             search_grid = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
         }
@@ -1418,7 +1425,9 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             // dependency index (leaf -> sides) and the writer list
             exclusive_scan(scnt.p, soff.p, m + 1, st);
             counters.zero();
-            k_writer_list<<<grid_for(m, BLK), BLK, 0, st>>>(m, status.p, writers.p, counters.p); ::tsr::note_launch();
+            DBuf<uint2> front(m, st), next(m, st);
+            k_writer_list<<<grid_for(m, BLK), BLK, 0, st>>>(m, status.p, keys.p, dleaf.p, writers.p, front.p,
+                                                            counters.p); ::tsr::note_launch();
             uint32_t cnt[2];
             TSR_CUDA(cudaMemcpyAsync(&cnt[0], soff.p + m, 4, cudaMemcpyDeviceToHost, st));
             TSR_CUDA(cudaMemcpyAsync(&cnt[1], counters.p, 4, cudaMemcpyDeviceToHost, st));
@@ -1437,19 +1446,18 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
                 k_segments<<<grid_for(nsens, BLK), BLK, 0, st>>>(nsens, ssorted.p, seg_lo.p, seg_hi.p); ::tsr::note_launch();
             }
             // waves: the frontier starts with every writer
-            DBuf<uint32_t> front(m, st), next(m, st), touched(m, st);
             uint32_t nf = nwri;
             if (nwri) {
-                TSR_CUDA(cudaMemcpyAsync(front.p, writers.p, (size_t)nwri * 4, cudaMemcpyDeviceToDevice, st));
-                DBuf<uint32_t> ctr(4, st);
+                DBuf<uint32_t> ctr(3, st);
                 ctr.zero();
                 uint32_t max_waves = max_waves_used;
-                uint32_t *fp = front.p, *np = next.p, *tp = touched.p, *kp = keys.p, *dp = dleaf.p, *mp = mark.p;
+                uint2 *fp = front.p, *np = next.p;
+                uint32_t *kp = keys.p, *dp = dleaf.p, *mp = mark.p;
                 uint32_t *slp = seg_lo.p, *shp = seg_hi.p, *blp = by_leaf.p, *up = unres.p, *cp = ctr.p;
                 uint32_t *wp = waves_total.p;
                 int *ep = derr.p;
-                void *args[] = {&nf, &fp, &np, &kp, &dp, &mp, &tp, &slp, &shp, &blp, &up, &cp, &max_waves, &wp, &ep};
-                TSR_CUDA(cudaLaunchCooperativeKernel((const void *)k_waves_coop, coop_grid, 256, args, 0, st));
+                void *args[] = {&nf, &fp, &np, &kp, &dp, &mp, &slp, &shp, &blp, &up, &cp, &max_waves, &wp, &ep};
+                TSR_CUDA(cudaLaunchCooperativeKernel((const void *)k_waves_coop, coop_grid, WAVE_THREADS, args, 0, st));
                 ::tsr::note_launch();
             }
             TSR_CUDA(cudaEventRecord(e2, st));
