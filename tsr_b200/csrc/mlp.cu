@@ -120,7 +120,7 @@ struct TrainShared {
     float w1[NF * NH], b1[NH], w2[NH * NH], b2[NH], w3[NH * NO], b3[NO + 2];   // as in the parameters (+ 2: alignment)
     float w2t[NH * LD];              // w2 transposed
     float h1[TR_ROWS * LD], h2[TR_ROWS * LD], d1[TR_ROWS * LD], d2[TR_ROWS * LD];
-    float x[TR_ROWS * 12], dout[TR_ROWS * NO];
+    float x[TR_ROWS * 12], dout[TR_ROWS * NO], warp_loss[TR_THREADS / 32];
 };
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
@@ -284,8 +284,14 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(uint32_t n, const floa
         add((t < 192 ? OB2 : OB1) + (t & 63), gb);
     }
     if (t < NO) add(OB3 + t, gb3);
+    // one addition to the loss a block: every one rounds at the size of the total
     for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((t & 31) == 0) atomicAdd(loss, l);
+    if ((t & 31) == 0) S.warp_loss[t >> 5] = l;
+    __syncthreads();
+    if (t == 0) {
+        for (int w = 1; w < TR_THREADS / 32; ++w) l += S.warp_loss[w];
+        atomicAdd(loss, l);
+    }
 }
 
 __global__ void k_adam(uint32_t np, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
