@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "handles.h"
+#include "limits.h"
 
 namespace cg = cooperative_groups;
 
@@ -890,26 +891,30 @@ __global__ void k_permute_samples(uint32_t n, uint32_t k, const uint32_t *old_of
 
 // -------------------------------------------------------------- neighbours
 // Leaves::getUnresponsibleEdgeNeighbor (Leaves.cpp:159-180) for every
-// (leaf, side); the edge event id is 6 * leaf + side.
+// (leaf, side); the edge event id is 6 * leaf + side.  The entry after the
+// rows' counts, row_count[nl], becomes the number of edges.
 __global__ void k_neighbor_events(uint32_t nl, const uint32_t *leaf_node, const D3 *leaf_min,
                                   const uint32_t *children, const D3 *nmin, const uint8_t *depth,
                                   const uint32_t *node_to_leaf, Root root, uint32_t *dst, uint32_t *row_count) {
     uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (uint64_t)nl * 6) return;
-    uint32_t l = e / 6, side = e % 6;
-    uint32_t node = leaf_node[l];
-    uint32_t maxd = depth[node];
-    double size = size_at(root.size, maxd);
-    D3 tp = side_center(leaf_min[l], size, side, dmul(0.5, size));
-    uint32_t nd;
-    uint32_t nb = get_node(children, nmin, root, tp, maxd, &nd);
     uint32_t out = INVALID;
-    if (nb != INVALID && children[nb] == INVALID && !(nd == maxd && nb < node)) out = node_to_leaf[nb];
-    dst[e] = out;
-    if (out != INVALID) {
-        atomicAdd(&row_count[l], 1u);
-        atomicAdd(&row_count[out], 1u);
+    if (e < (uint64_t)nl * 6) {
+        uint32_t l = e / 6, side = e % 6;
+        uint32_t node = leaf_node[l];
+        uint32_t maxd = depth[node];
+        double size = size_at(root.size, maxd);
+        D3 tp = side_center(leaf_min[l], size, side, dmul(0.5, size));
+        uint32_t nd;
+        uint32_t nb = get_node(children, nmin, root, tp, maxd, &nd);
+        if (nb != INVALID && children[nb] == INVALID && !(nd == maxd && nb < node)) out = node_to_leaf[nb];
+        dst[e] = out;
+        if (out != INVALID) {
+            atomicAdd(&row_count[l], 1u);
+            atomicAdd(&row_count[out], 1u);
+        }
     }
+    const int edges = __syncthreads_count(out != INVALID);
+    if (threadIdx.x == 0 && edges) atomicAdd(&row_count[nl], (uint32_t)edges);
 }
 
 // Both ends of every edge into their rows, in no order yet: (event, other end).
@@ -1630,8 +1635,10 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
                                                             t.depth.p, t.node_to_leaf.p, root, dst.p, rowc.p); ::tsr::note_launch();
         t.nb_off.alloc(nl + 1, st);
         exclusive_scan(rowc.p, t.nb_off.p, nl + 1, st);
-        // two entries an edge: 12 per leaf at most, and the offsets are 32-bit, as the events are
-        const uint32_t nent = read_scalar(t.nb_off.p + nl, st);
+        // the edges number at most the events, so their 32-bit count is exact; the rows' total may not be
+        uint32_t nent = 0;
+        if (!neighbor_entries(read_scalar(rowc.p + nl, st), &nent))
+            fail(TSR_ERR_OVERFLOW_U32, "too many neighbour entries for 32-bit row offsets");
         t.n_nb = nent;
         DBuf<uint2> entries(nent, st);
         t.nbs.alloc(nent, st);
