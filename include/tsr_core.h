@@ -112,7 +112,9 @@ typedef struct {
     uint64_t accepted_emptiness;       /* ... EMPTINESS pass */
     uint64_t visited_sampleness;       /* tree nodes tested against a cone, SAMPLENESS pass */
     uint64_t visited_emptiness;        /* ... EMPTINESS pass */
-    uint64_t visited_priors;           /* tree nodes classified by the prior sphere queries */
+    uint64_t visited_priors;           /* tree nodes classified by the prior sphere queries, once for each query:
+                                          eight per children block a query opens (the queries of a block's leaves
+                                          are answered together and open the same blocks) */
     uint64_t pruned_leaves;            /* prior queries the pruned field skipped (0 for the plain field) */
     uint64_t repaired_leaves;          /* skipped positive leaves queried after all: next to a negative leaf, side of EPSILON unproved */
     uint64_t certified_leaves;         /* skip candidates whose sign bounds of their prior proved */

@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
 #pragma unroll
             for (int q = 0; q < 8; ++q) uE[q] = uS[q] = 0.0;
         }
-        uint32_t tested = 0;
+        uint32_t opened = sp | waiting;   // children blocks
         __syncwarp();
         // whole-numbered distances: undecided only when zero
         const bool whole = in.whole_radius && !in.deep && 4.0f * ru * P.ea < 0.125f;
@@ -1163,7 +1163,6 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
                                     aS[q] += v[k].y / PP_UNIT;
                                 }
                     }
-                    tested += 64;
                     waiting -= 8;
                 } while ((waiting >= 8 || (waiting > 0 && sp == 0)) && ties <= PP_TIES - 64);
                 if (waiting < 0) waiting = 0;
@@ -1175,7 +1174,6 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
             const bool valid = quarter < take;
             const uint32_t b = w.stack[sp - 1 - (valid ? quarter : 0)], node = 1 + 8 * b + ci;
             sp -= take;
-            tested += 8 * take;
             const uint2 r = __ldg(&in.rec[node + REC_OFFSET]);
             const float4 B = __ldg(&in.blocks[b]);
             bool next = false;
@@ -1235,6 +1233,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
             const uint32_t block = (r.x - 1) >> 3;
             const bool push = next && (r.y & REC_HAS_INNER), wait = next && (r.y & REC_HAS_LEAVES);
             const unsigned pm = __ballot_sync(FULL, push), wm = __ballot_sync(FULL, wait);
+            opened += __popc(pm | wm);
             if (sp + __popc(pm) > PP_STACK) {
                 if (lane == 0) atomicExch(err, 2);   // deeper than any tree
             } else {
@@ -1249,7 +1248,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
             waiting += __popc(wm);
             __syncwarp();
         }
-        nvis += (unsigned long long)tested * __popc(mask);
+        nvis += 8ull * opened * __popc(mask);   // every node of an opened block, for each of the queries
         allE = warp_sum(allE);
         allS = warp_sum(allS);
         double E = 0.0, S = 0.0, UE = 0.0, US = 0.0;
