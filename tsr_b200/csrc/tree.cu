@@ -263,7 +263,8 @@ struct SideF {
         const float r = (float)q.r;
         r2 = r * r;
         e = 3e-6f * reach + margin;
-        e_plane = 2.0f * (n_hi - n_lo) * e;
+        // 1e-25: the products of a very short normal round to FP32's subnormals, by up to 2^-149 x reach each
+        e_plane = fmaf(2.0f * (n_hi - n_lo), e, 1e-25f);
         positive = q.positive;
     }
     // d2 against r2, each with its rounding; t = the sum of the terms squared
