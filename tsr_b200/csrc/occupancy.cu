@@ -1233,7 +1233,6 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
             const uint32_t block = (r.x - 1) >> 3;
             const bool push = next && (r.y & REC_HAS_INNER), wait = next && (r.y & REC_HAS_LEAVES);
             const unsigned pm = __ballot_sync(FULL, push), wm = __ballot_sync(FULL, wait);
-            opened += __popc(pm | wm);
             if (sp + __popc(pm) > PP_STACK) {
                 if (lane == 0) atomicExch(err, 2);   // deeper than any tree
             } else {
@@ -1246,6 +1245,7 @@ __global__ void __launch_bounds__(32 * PP_WARPS, BOUNDS ? 3 : TSR_PRIOR_BLOCKS)
                 w.leaf_box[j] = corner;
             }
             waiting += __popc(wm);
+            opened += __popc(pm | wm);
             __syncwarp();
         }
         nvis += 8ull * opened * __popc(mask);   // every node of an opened block, for each of the queries
