@@ -221,8 +221,9 @@ void triangulate_depth(const double *depths_host, uint32_t W, uint32_t H, const 
     cudaStream_t st = m.stream;
     const uint64_t np64 = (uint64_t)W * H;
     if (W < 2 || H < 2) fail(TSR_ERR_INVALID_ARG, "a depth map needs at least 2 x 2 pixels");
-    // up to 2 triangles per pixel and 6 neighbour events per triangle stay below 2^32
-    if (12 * np64 >= NONE) fail(TSR_ERR_OVERFLOW_U32, "depth map too large for 32-bit neighbour event indices");
+    // up to 2 triangles, so 6 corners, per pixel: their 32-bit indices would hold twice this
+    // limit, which is the one that callers know
+    if (12 * np64 >= NONE) fail(TSR_ERR_OVERFLOW_U32, "depth map too large: 2^32 / 12 pixels at most");
     const uint32_t np = (uint32_t)np64, nblocks = (W - 1) * (H - 1);
     Mat3 Mvs, Mws;
     for (int i = 0; i < 9; ++i) {
@@ -274,7 +275,8 @@ void triangulate_depth(const double *depths_host, uint32_t W, uint32_t H, const 
     angle_weighted_normals(m.tris.p, nt, m.vpos.p, nv, m.vnrm.p, st);
     // ---- scales: the mean distance to the neighbours
     if (nv) {
-        k_vertex_scales<<<grid_for(np, BLK), BLK, 0, st>>>(W, H, code.p, m.pix2v.p, m.vpos.p, m.vscale.p); ::tsr::note_launch();
+        k_vertex_scales<<<grid_for(np, BLK), BLK, 0, st>>>(W, H, code.p, m.pix2v.p, m.vpos.p, m.vscale.p);
+        ::tsr::note_launch();
     }
     TSR_CUDA(cudaStreamSynchronize(st));
     TSR_CUDA(cudaGetLastError());

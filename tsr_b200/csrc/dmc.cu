@@ -197,7 +197,8 @@ void extract_dmc(const tsr_tree &t, const tsr_occupancy &o, tsr_mesh &m) {
     DBuf<uint64_t> keys(mc, st), skeys(mc, st);
     DBuf<uint32_t> vals(mc, st), svals(mc, st), ends(2ull * mc, st);
     const int leaf_bits = bits_below(t.n_leaves);
-    k_emit<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, t.cells.p, o.occ.p, toff.p, leaf_bits, keys.p, vals.p, ends.p); ::tsr::note_launch();
+    k_emit<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, t.cells.p, o.occ.p, toff.p, leaf_bits, keys.p, vals.p, ends.p);
+    ::tsr::note_launch();
     sortp(keys.p, skeys.p, vals.p, svals.p, mc, 2 * leaf_bits, st);
     DBuf<uint32_t> head(mc, st), segid(mc, st), first(mc, st);
     k_heads<<<grid_for(mc, BLK), BLK, 0, st>>>(mc, skeys.p, svals.p, head.p, first.p); ::tsr::note_launch();

@@ -459,7 +459,8 @@ void postprocess_mesh(tsr_mesh &m, uint32_t min_isle_size, tsr_mesh_post_counts 
         const int vertex_bits = bits_for(nv - 1);   // edges have vertices
         k_edge_keys<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, m.tris.p, vertex_bits, keys.p, vals.p); ::tsr::note_launch();
         sort_kv(keys.p, skeys.p, vals.p, svals.p, nc, 2 * vertex_bits, st);
-        k_edge_runs<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, skeys.p, vertex_bits, svals.p, border.p, parent.p, err.p); ::tsr::note_launch();
+        k_edge_runs<<<grid_for(nc, BLK), BLK, 0, st>>>(nc, skeys.p, vertex_bits, svals.p, border.p, parent.p, err.p);
+        ::tsr::note_launch();
     }
     if (nv) {
         k_labels<<<grid_for(nv, BLK), BLK, 0, st>>>(nv, parent.p, label.p, size.p, err.p); ::tsr::note_launch();

@@ -110,7 +110,7 @@ __global__ void k_feature_minmax(uint32_t nl, const int *rmin, const int *rmax, 
 //
 // A batch of 8192 rows: 84 us with a thread per row (two warps an SM, every
 // operand a scalar load of its own) -> 24 us; 3.2 us of FP32 arithmetic at
-// the peak.  What bounds it is shared memory bandwidth and the ten barriers of
+// the peak.  What bounds it is shared memory bandwidth and the seven barriers of
 // a tile.
 constexpr int TR_ROWS = 64;
 constexpr int TR_THREADS = 256;
@@ -185,7 +185,8 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(uint32_t n, const floa
             }
             for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<float4 *>(&S.h1[(4 * ty + i) * LD + 4 * tx]) =
-                    make_float4(fmaxf(acc[i][0], 0.0f), fmaxf(acc[i][1], 0.0f), fmaxf(acc[i][2], 0.0f), fmaxf(acc[i][3], 0.0f));
+                    make_float4(fmaxf(acc[i][0], 0.0f), fmaxf(acc[i][1], 0.0f), fmaxf(acc[i][2], 0.0f),
+                                fmaxf(acc[i][3], 0.0f));
         }
         __syncthreads();
         {   // h2 = relu(h1 w2 + b2)
@@ -195,7 +196,8 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(uint32_t n, const floa
             tile_product<NH>(S.h1, S.w2, tx, ty, acc);
             for (int i = 0; i < 4; ++i)
                 *reinterpret_cast<float4 *>(&S.h2[(4 * ty + i) * LD + 4 * tx]) =
-                    make_float4(fmaxf(acc[i][0], 0.0f), fmaxf(acc[i][1], 0.0f), fmaxf(acc[i][2], 0.0f), fmaxf(acc[i][3], 0.0f));
+                    make_float4(fmaxf(acc[i][0], 0.0f), fmaxf(acc[i][1], 0.0f), fmaxf(acc[i][2], 0.0f),
+                                fmaxf(acc[i][3], 0.0f));
         }
         __syncthreads();
         {   // outputs, loss and its gradient: two threads an output, half of the inner dimension each
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(uint32_t n, const floa
                                 h.z > 0.0f ? acc[i][2] : 0.0f, h.w > 0.0f ? acc[i][3] : 0.0f);
             }
         }
-        // w2: rows of w2 4 ty .., columns 4 tx ..; the other half of the block's threads take w3, b2, b1 below
+        // w2: rows 4 ty .., columns 4 tx .. by every thread
 #pragma unroll 4
         for (int r = 0; r < TR_ROWS; ++r) {
             const float4 a = *reinterpret_cast<const float4 *>(&S.h1[r * LD + 4 * ty]);
@@ -254,7 +256,8 @@ __global__ void __launch_bounds__(TR_THREADS) k_mlp_train(uint32_t n, const floa
                 for (int j = 0; j < 4; ++j) g2[i][j] = fmaf(aa[i], bb[j], g2[i][j]);
         }
         __syncthreads();
-        // w1[f][h]: h = t % 64, f = t / 64 + 0, 4, 8; w3[j][k] by threads 0..127; b2 and b1 by the others
+        // w1[f][h] by every thread: h = t % 64, f = t / 64 + 0, 4 and, below thread 128, 8;
+        // w3[j][k] by threads 0..127; b2 by 128..191, b1 by 192..255; b3 by threads 0 and 1
 #pragma unroll 8
         for (int r = 0; r < TR_ROWS; ++r) {
             const float d = S.d1[r * LD + (t & 63)];
@@ -374,6 +377,11 @@ __global__ void k_mlp_pack_frags(const float *P, uint32_t *frag) {
 }
 
 // Logits of n rows of normalized features; each warp takes 16 rows at a time.
+//
+// 2M rows take 95 us: 19 clocks an mma.sync and scheduler, where a loop of
+// nothing else reaches 8.7.  No unit is full (tensor pipe 46 %, shared memory's
+// data path 72 %, issue 53 %): with six and a half warps a scheduler, 1.5 ready
+// on average, it waits for the fragments' loads and the products they feed.
 __global__ void __launch_bounds__(128) k_mlp_infer(uint32_t n, const float *x, const uint32_t *frag_g,
                                                  const float *params, float *out) {
     __shared__ uint32_t frag[NFRAG];

@@ -11,9 +11,10 @@
 // cone count are FP64 (as the reference's Real = double); kernel evaluation
 // runs in FP32 in a frame centred on the sample, and every per-leaf sum is an
 // FP64 accumulator updated by FP64 atomic adds whose result is not used (no
-// round trip per accepted pair).  Priors and occupancy are evaluated in FP64;
-// the prior's sphere / box membership test is the same FP64 expression as the
-// tree build's, so the set of leaves each prior sums over is exact.
+// round trip per accepted pair).  Priors and occupancy are evaluated in FP64.
+// Which leaves a prior sums is decided by FP32 distances where those are certain
+// (exact on the lattice of box corners, or outside their error bound) and by the
+// tree build's FP64 expression everywhere else, so the set is exact.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -105,9 +106,11 @@ __device__ __forceinline__ void cone_coords(const ConeF &c, F3 x, float &te, F3 
     axis_offset(c, u, te, q, r2);
 }
 
-// The same for the centre of child ci of a traversed node.  Its te is rounded
-// as it always was: unfused products in the SAMPLENESS pass, and in the
-// EMPTINESS pass a fused last product for the first five children only.
+// The same for the centre of child ci of a traversed node.  Unfused products in
+// the SAMPLENESS pass, and in the EMPTINESS pass a fused last product for the
+// first five children only: no numerical reason, the two are equally accurate,
+// but this is how the kernel that defined the field's values was rounded, and a
+// field keeps its values, bit for bit per link, from one version to the next.
 template <int TYPE>
 __device__ __forceinline__ void child_coords_of(const ConeF &c, uint32_t ci, F3 x, float &te, F3 &q, float &r2) {
     const F3 u = x - c.end;
@@ -429,12 +432,12 @@ __global__ void __launch_bounds__(128) k_link_setup(uint64_t nlinks, const uint3
 //
 // Measured, SAMPLENESS + EMPTINESS pass: 14 + 24 -> 2.3 + 5.3 ms at 300k
 // held-out samples, 20 + 30 -> 15 + 27 ms at 4M CSG, 99 + 247 -> 59 + 190 ms
-// at 16M held-out.  What bounds it is instruction issue (3.2 of 4 a clock); the
-// FP64 atomics keep their L2 units 8 % busy.
+// at 16M held-out.  What bounds it is instruction issue (3.2 of 4 a clock).
 //
 // The FP32 arithmetic of a child's box is part of the result, so it follows
 // one rule: the first surviving child's corner comes from its parent's by the
-// FP32 recurrence, every other one's from the FP64 tree.
+// FP32 recurrence, every other one's from the FP64 tree.  Like the rounding in
+// child_coords_of it keeps a link's values what they were; it carries no accuracy.
 //
 // Leaf flags are not written here: a leaf got a kernel exactly when its sum is
 // non-zero (every accepted value is >= EPSILON), so they are set afterwards
@@ -477,13 +480,14 @@ __device__ __forceinline__ ConeF cone_of(const float4 *l) {
 
 template <int TYPE>
 __global__ void __launch_bounds__(32 * CX_WARPS, TSR_CONE_BLOCKS)
-    k_cones(uint64_t nlinks, uint32_t per, uint32_t stack, uint32_t warp_bytes, const LinkRec *links, TreeIn tr, const uint2 *rec, float root_size_f,
-            double *ksum, double *clen, unsigned long long *accepted, unsigned long long *next_link,
-            unsigned long long *visits, int *err, double sign) {
+    k_cones(uint64_t nlinks, uint32_t per, uint32_t stack, uint32_t warp_bytes, const LinkRec *links, TreeIn tr,
+            const uint2 *rec, float root_size_f, double *ksum, double *clen, unsigned long long *accepted,
+            unsigned long long *next_link, unsigned long long *visits, int *err, double sign) {
     const unsigned FULL = 0xffffffffu;
     extern __shared__ float4 cone_shared[];
     __shared__ float sizes[64];     // edge length of a node at a depth
-    ConeWarp &w = *reinterpret_cast<ConeWarp *>(reinterpret_cast<char *>(cone_shared) + (threadIdx.x >> 5) * warp_bytes);
+    ConeWarp &w =
+        *reinterpret_cast<ConeWarp *>(reinterpret_cast<char *>(cone_shared) + (threadIdx.x >> 5) * warp_bytes);
     float4 *const stack_box = w.box;
     uint16_t *const stack_tag = reinterpret_cast<uint16_t *>(w.box + stack);
     const unsigned lane = threadIdx.x & 31, below = (1u << lane) - 1u, ci = lane & 7u;
@@ -830,7 +834,11 @@ struct PriorIn {
     bool whole_radius;          // eight radii are a whole number, small enough for exact FP32 squares
 };
 
-constexpr int PP_STACK = 28 * MAX_TREE_DEPTH + 32;   // a step pops four blocks and pushes at most 32
+// A step pops four blocks and pushes at most 32.  What one step pushed lies below
+// only what came of its own blocks, at least a level deeper, so the steps with
+// blocks left are at most one a depth; each but the last has lost four of its 32
+// to the step right after it.
+constexpr int PP_STACK = 28 * MAX_TREE_DEPTH + 32;
 constexpr int PP_LEAVES = 64;   // blocks whose leaves wait; worked off when fewer than 32 are free
 constexpr int PP_TIES = 96;     // leaves that touch a sphere; worked off when fewer than 64 are free
 constexpr int PP_WARPS = 4;
@@ -867,9 +875,10 @@ constexpr int PP_WARPS = 4;
 // psum rows of its own per expansion, 128 + 256 cache lines a warp's step, and
 // the L1 passed 0.7 child tests a clock and SM; here the lines are shared and a
 // test costs 12 of a lane's instructions.  What bounds it is latency at four
-// warps a scheduler (126 registers, 32 of them the sums): two leaves a lane at a
+// warps a scheduler (128 registers, 32 of them the sums): two leaves a lane at a
 // time are 8 % faster than one, three warps 23 % slower, five spill.  The eight
-// spheres test 1.6 times the boxes one does.
+// spheres together open the blocks that any of them needs: 1.6 times the nodes
+// are classified for each (23.5k against 14.4k a leaf at 16M held-out samples).
 //
 // BOUNDS (the pruned field's sign certificates): a node that straddles a
 // query's sphere at depth >= the query leaf's depth - coarse_up is not
@@ -1285,7 +1294,6 @@ __global__ void k_prior_root(const double2 *psum, double *prior, double2 *bounds
     else prior[0] = p;
 }
 
-// Occupancy::getOccupancy (Occupancy.cpp:570-587), FP64.
 // Occupancy::getOccupancy (Occupancy.cpp:570-587), FP64.  In a pruned field
 // (pred != null) a reliable leaf whose prior was not queried (need == 0)
 // gets its sign from E == 0 / S == 0 or from the pruner, and the value
@@ -1437,8 +1445,9 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
                                                                         ssum, slen, cone_count.p, accepted.p + 1,
                                                                         sign);
         ::tsr::note_launch();
-        k_cones<SAMPLENESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, ssum, slen,
-                                                         accepted.p + 1, next_link.p, accepted.p + 3, err.p, sign);
+        k_cones<SAMPLENESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(
+            nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, ssum, slen,
+            accepted.p + 1, next_link.p, accepted.p + 3, err.p, sign);
         ::tsr::note_launch();
     }
     // flags mark leaves that received a kernel; removal leaves them set (Occupancy.cpp:232)
@@ -1481,8 +1490,9 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
         k_link_setup<EMPTINESS><<<grid_for(nlinks, 128), 128, 0, st>>>(nlinks, order.p, in, tr, recs.p, lrec.p, esum,
                                                                        elen, cone_count.p, accepted.p, sign);
         ::tsr::note_launch();
-        k_cones<EMPTINESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, esum, elen,
-                                                        accepted.p, next_link.p, accepted.p + 2, err.p, sign);
+        k_cones<EMPTINESS><<<x_grid, 32 * CX_WARPS, cone_smem, st>>>(
+            nlinks, links_per_warp, stack, warp_bytes, lrec.p, tr, recs.p, (float)t.root_size, esum, elen, accepted.p,
+            next_link.p, accepted.p + 2, err.p, sign);
         ::tsr::note_launch();
     }
     if (sign > 0.0) {
@@ -1505,16 +1515,18 @@ void compute_occupancy(const tsr_tree &t, const tsr_cameras_view &cv, const tsr_
     for (int d = (int)t.level_start.size() - 2; d >= 0; --d) {
         uint32_t lo = t.level_start[d], hi = t.level_start[d + 1];
         k_prior_sums<<<grid_for(hi - lo, BLK), BLK, 0, st>>>(lo, hi, nn, t.level_order.p, t.children.p,
-                                                            t.node_to_leaf.p, o.states.p, elen, slen, psum.p, err.p + 1); ::tsr::note_launch();
+                                                            t.node_to_leaf.p, o.states.p, elen, slen, psum.p,
+                                                            err.p + 1); ::tsr::note_launch();
     }
     const uint32_t nb = (nn - 1) / 8;
     DBuf<float4> block_corners(nb, st);
     DBuf<uint32_t> block_order = depth_ordered_blocks(nb, t.depth.p, st);
     if (nb) {
-        k_block_corners<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, t.parents.p, t.depth.p, block_corners.p); ::tsr::note_launch();
+        k_block_corners<<<grid_for(nb, BLK), BLK, 0, st>>>(nb, t.parents.p, t.depth.p, block_corners.p);
+        ::tsr::note_launch();
     }
-    PriorIn pin{nn, t.parents.p, t.nmin.p, recs.p, block_corners.p, psum.p, err.p + 1, t.root_size, p.relative_radius_for_priors,
-                0.0, t.max_depth >= LATTICE_DEPTH, false};
+    PriorIn pin{nn, t.parents.p, t.nmin.p, recs.p, block_corners.p, psum.p, err.p + 1, t.root_size,
+                p.relative_radius_for_priors, 0.0, t.max_depth >= LATTICE_DEPTH, false};
     {
         // a corner is a sum of at most MAX_TREE_DEPTH steps, a centre one more, each rounded to half an ulp
         double m = 0.0;

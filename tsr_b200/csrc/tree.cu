@@ -559,7 +559,8 @@ __global__ void __launch_bounds__(128) k_search(uint32_t m, const uint32_t *side
                         have = false;
                     } else {
                         if (ci == 0)
-                            st[sp] = (uint64_t)c0 | ((uint64_t)rest << 32) | ((uint64_t)rel << 40) | ((uint64_t)d << 48);
+                            st[sp] = (uint64_t)c0 | ((uint64_t)rest << 32) | ((uint64_t)rel << 40) |
+                                     ((uint64_t)d << 48);
                         ++sp;
                     }
                 }
@@ -615,9 +616,9 @@ constexpr uint32_t WAVE_THREADS = 1024;
 // dependent loads and atomics and the barrier, whose cost grows with the
 // blocks: one block of 1024 threads a SM instead of eight of 256, and a warp a
 // pair (a leaf's list is long: 8 lanes 9.4, 16 lanes 7.9, 32 lanes 7.2 ms of
-// resolution at 4M CSG samples).  Measured, a wave 20 -> 10 us there (471
-// waves in 20 rounds, resolution 12.1 -> 7.2 ms), 9.9 -> 7.4 ms at 16M held-out
-// samples.  Two blocks a SM, or two sides a lane at a time, give nothing.
+// resolution at 4M CSG samples).  Measured, a wave 20 -> 10 us there (a scene
+// with 471 waves in 20 rounds, resolution 12.1 -> 7.2 ms), 9.9 -> 7.4 ms at 16M
+// held-out samples.  Two blocks a SM, or two sides a lane at a time, give nothing.
 __global__ void __launch_bounds__(WAVE_THREADS)
     k_waves_coop(uint32_t nf0, uint2 *front, uint2 *next, const uint32_t *keys, const uint32_t *dleaf, uint32_t *mark,
                  const uint32_t *seg_lo, const uint32_t *seg_hi, const uint32_t *by_leaf, uint32_t *unres,
@@ -1116,8 +1117,9 @@ __global__ void k_frames_count(uint32_t m, const uint8_t *type, const uint32_t *
 
 __global__ void k_frames_write(uint32_t m, const uint8_t *type, const uint32_t *nodes, const uint64_t *khi,
                                const uint64_t *klo, uint32_t level, const uint32_t *children,
-                               const uint32_t *node_to_leaf, const uint64_t *offsets, uint32_t cbase, uint8_t *otype, uint32_t *onodes, uint64_t *okhi, uint64_t *oklo,
-                               uint32_t *cells, uint64_t *ckhi, uint64_t *cklo) {
+                               const uint32_t *node_to_leaf, const uint64_t *offsets, uint32_t cbase,
+                               uint8_t *otype, uint32_t *onodes, uint64_t *okhi, uint64_t *oklo, uint32_t *cells,
+                               uint64_t *ckhi, uint64_t *cklo) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     uint32_t fo = (uint32_t)offsets[i], co = cbase + (uint32_t)(offsets[i] >> 32);
@@ -1425,8 +1427,8 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
                                                            dleaf.p, margin, derr.p); ::tsr::note_launch();
             taken.zero();
             k_search<false><<<std::min(search_grid, grid_for(m, 16)), 128, 0, st>>>(
-                m, nullptr, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p, status.p, witness.p, scnt.p, nullptr,
-                nullptr, nullptr, margin, taken.p, derr.p); ::tsr::note_launch();
+                m, nullptr, keys.p, v, root, pos.p, nrm.p, scale.p, h_svo, begin.p, status.p, witness.p, scnt.p,
+                nullptr, nullptr, nullptr, margin, taken.p, derr.p); ::tsr::note_launch();
             TSR_CUDA(cudaEventRecord(e1, st));
             // dependency index (leaf -> sides) and the writer list
             exclusive_scan(scnt.p, soff.p, m + 1, st);
@@ -1645,8 +1647,10 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
         t.nbs.alloc(nent, st);
         rowc.zero();
         if (nent) {
-            k_neighbor_entries<<<grid_for(ne, BLK), BLK, 0, st>>>(ne, dst.p, t.nb_off.p, rowc.p, entries.p); ::tsr::note_launch();
-            k_neighbor_rows<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, t.nb_off.p, entries.p, t.nbs.p); ::tsr::note_launch();
+            k_neighbor_entries<<<grid_for(ne, BLK), BLK, 0, st>>>(ne, dst.p, t.nb_off.p, rowc.p, entries.p);
+            ::tsr::note_launch();
+            k_neighbor_rows<<<grid_for(nl, BLK), BLK, 0, st>>>(nl, t.nb_off.p, entries.p, t.nbs.p);
+            ::tsr::note_launch();
         }
     }
     t.stage_ms[4] = timer.lap();
@@ -1715,7 +1719,8 @@ void build_tree(tsr_tree &t, const tsr_samples_view &sv, bool on_device) {
             const bool deep = levels > 12;
             if (deep) {
                 sort_pairs(all_lo.p, k2.p, idx.p, idx2.p, ncells, st, 64, 64 - 5 * ((int)levels - 12));
-                k_gather_u64<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx2.p, all_hi.p, k3.p); ::tsr::note_launch();
+                k_gather_u64<<<grid_for(ncells, BLK), BLK, 0, st>>>(ncells, idx2.p, all_hi.p, k3.p);
+                ::tsr::note_launch();
                 sort_pairs(k3.p, k2.p, idx2.p, idx3.p, ncells, st, 64, 4);
             } else {
                 sort_pairs(all_hi.p, k2.p, idx.p, idx3.p, ncells, st, 64, 64 - 5 * (int)levels);
